@@ -1,0 +1,76 @@
+"""The solver's kernels at the edges of their thread layouts: set counts that
+do and do not divide a block, several threads to a row (1, 2 and 4 sets), a
+single row, rows without entries, lower-triangle and full patterns."""
+import numpy as np
+import pytest
+
+from symboliclib_gb300 import native
+
+pytestmark = pytest.mark.gpu
+
+
+def pattern(n, density, lower, rng, diagonal=True):
+    """CSC pattern of a random symmetric matrix (lower triangle or full)."""
+    m = rng.random((n, n)) < density
+    m = np.tril(m | m.T)
+    np.fill_diagonal(m, diagonal)
+    if not lower:
+        m = m | m.T
+    cp = np.concatenate([[0], np.cumsum(m.sum(0))])
+    return cp, np.concatenate([np.flatnonzero(m[:, j]) for j in range(n)]).astype(np.int32)
+
+
+def dense(n, cp, ri, v, lower):
+    A = np.zeros((n, n))
+    for j in range(n):
+        A[ri[cp[j]:cp[j + 1]], j] = v[cp[j]:cp[j + 1]]
+    return A + np.tril(A, -1).T if lower else A
+
+
+@pytest.mark.parametrize("n", [1, 37, 400])
+@pytest.mark.parametrize("sets", [1, 2, 3, 4, 5, 8, 33, 100, 129, 256])
+@pytest.mark.parametrize("lower", [True, False])
+def test_multiply(n, sets, lower):
+    """|q - A p| <= (terms of a row) 2^-53 |A| |p| with room for either summation order."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(n * 1000 + sets)
+    cp, ri = pattern(n, 0.08, lower, rng, diagonal=n == 1)
+    if not len(ri):
+        return
+    v, p = rng.standard_normal((sets, len(ri))), rng.standard_normal((sets, n))
+    q = torch.full((sets, n), np.nan, dtype=torch.float64, device="cuda")
+    native.SparseSolver(n, cp, ri, lower, sets).multiply(torch.from_numpy(v).cuda(), torch.from_numpy(p).cuda(), q)
+    q = q.cpu().numpy()
+    for s in {0, sets // 2, sets - 1}:
+        A = dense(n, cp, ri, v[s], lower)
+        assert np.all(np.abs(q[s] - A @ p[s]) <= 2 * n * 2.0 ** -53 * (np.abs(A) @ np.abs(p[s])))
+
+
+@pytest.mark.parametrize("method,block", [(native.SOLVER_CG, 1), (native.SOLVER_BICGSTAB, 1),
+                                          (native.SOLVER_BICGSTAB, 2), (native.SOLVER_BICGSTAB, 4)])
+@pytest.mark.parametrize("n,sets", [(4, 1), (36, 2), (36, 7), (400, 4), (400, 40), (20, 256)])
+def test_solve_diagonally_dominant(n, sets, method, block):
+    """Condition number at most 1.5 * 3 (Gershgorin discs around uneven
+    diagonals within a factor 3, radius a fifth), residual 1e-12: the solution to 1e-11."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(n + sets)
+    cp, ri = pattern(n, 0.1, True, rng)
+    v = rng.uniform(-1.0, 1.0, (sets, len(ri)))
+    col = np.repeat(np.arange(n), np.diff(cp))
+    off = ri != col
+    for s in range(sets):
+        row = np.bincount(ri[off], np.abs(v[s, off]), n) + np.bincount(col[off], np.abs(v[s, off]), n)
+        v[s, off] *= 0.2 / max(row.max(), 1.0) if off.any() else 1.0
+        v[s, ~off] = rng.uniform(1.0, 3.0, n)
+    b = rng.standard_normal((sets, n))
+    solver = native.SparseSolver(n, cp, ri, True, sets)
+    for stride in ([1] if block == 1 else [1, n // block]):
+        if block > 1:
+            solver.set_block_preconditioner(block, stride)
+        x = torch.full((sets, n), np.nan, dtype=torch.float64, device="cuda")
+        it, res = solver.solve(torch.from_numpy(v).cuda(), torch.from_numpy(b).cuda(), x, tol=1e-12, max_iter=64,
+                               method=method)
+        assert res <= 1e-12
+        for s in {0, sets - 1}:
+            ref = np.linalg.solve(dense(n, cp, ri, v[s], True), b[s])
+            assert np.linalg.norm(x[s].cpu().numpy() - ref) <= 1e-11 * np.linalg.norm(ref)
