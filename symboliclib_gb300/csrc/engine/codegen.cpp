@@ -56,9 +56,10 @@ const char* libName(int op) {
 }
 
 // Emits the device function evaluating kernel k.
-//   Strided items (grouped == nullptr): symgbBody<k><L2>(..., i, s) evaluates
-//     one work item (instance i, value set s) and loads its own index and
-//     constant entries.
+//   Strided items (grouped == nullptr): symgbBody<k><L2, ORDER>(..., i, s)
+//     evaluates one work item (instance i, value set s) and loads its own index
+//     and constant entries; ORDER is what it does between these loads, which
+//     no kernel writes, and its first read of x (launchOrder).
 //   Grouped items: symgbGroup<k><L2, IT, FULL>(..., g, s) evaluates the IT
 //     consecutive instances g*IT .. g*IT+IT-1 of value set s; each index and
 //     constant row is read with one vector load from the padded copies of the
@@ -84,7 +85,7 @@ std::size_t emitBody(std::ostringstream& os, int k, const symgb_kernel_desc& d, 
               "const double* __restrict__ c, double* __restrict__ res, const unsigned* __restrict__ dp, "
               "unsigned long long g, unsigned s) {\n";
     else
-        os << "template <int L2>\n__device__ __forceinline__ void symgbBody" << k
+        os << "template <int L2, int ORDER = 0>\n__device__ __forceinline__ void symgbBody" << k
            << "(const double* SYMGB_XR x, double* SYMGB_XR xw, const unsigned* __restrict__ p, "
               "const double* __restrict__ c, double* __restrict__ res, const unsigned* __restrict__ dp, "
               "unsigned long long i, unsigned s) {\n";
@@ -121,7 +122,20 @@ std::size_t emitBody(std::ostringstream& os, int k, const symgb_kernel_desc& d, 
                << " + i);\n";
     }
     std::vector<int> constVar;
-    if (g) {
+    if (!g) {
+        constVar.assign(d.num_constant_rows, -1);
+        int consts = 0;
+        for (std::uint64_t w : loads) {
+            if ((int)(w & 0xff) != OP_LDC) continue;
+            const std::uint32_t row = (std::uint32_t)(w >> 32);
+            if (row >= d.num_constant_rows) throw std::runtime_error("codegen: constant row out of range");
+            if (constVar[row] >= 0) continue;
+            constVar[row] = consts++;
+            os << "    const double k" << constVar[row] << " = SYMGB_LD(c + "
+               << u64(d.constants_offset + (std::uint64_t)row * n) << " + i);\n";
+        }
+        os << "#ifdef SYMGB_ORDERED\n    x = symgbOrder<ORDER>(x);\n#endif\n";
+    } else {
         constVar.assign(d.num_constant_rows, -1);
         int consts = 0;
         for (std::uint64_t w : loads) {
@@ -148,11 +162,7 @@ std::size_t emitBody(std::ostringstream& os, int k, const symgb_kernel_desc& d, 
                << " + " << imm << "u)" << xs << ");\n";
         } else if (op == OP_LDC) {
             const std::string v = fresh(dst);
-            if (g)
-                os << in << "const double " << v << " = k" << constVar[imm] << "[j];\n";
-            else
-                os << in << "const double " << v << " = SYMGB_LD(c + "
-                   << u64(d.constants_offset + (std::uint64_t)imm * n) << " + i);\n";
+            os << in << "const double " << v << " = k" << constVar[imm] << (g ? "[j];\n" : ";\n");
         } else {
             throw std::runtime_error("codegen: unknown load word");
         }
@@ -225,21 +235,22 @@ constexpr std::size_t kSplitOps = 1024;
 // loads are in flight together.  `split`: threads whose items are all in
 // range take an unguarded copy of the loop (kSplitOps).
 void emitItems(std::ostringstream& os, int k, std::uint64_t total, unsigned S, int tpb, int items, int l2,
-               const std::string& b0, const char* indent, bool split) {
+               const std::string& b0, const char* indent, bool split, int order) {
+    const std::string targs = "<" + std::to_string(l2) + (order ? ", " + std::to_string(order) : std::string()) + ">";
     os << indent << "const unsigned long long w0 = (" << b0 << ") * " << (std::uint64_t)tpb * items
        << "ull + threadIdx.x;\n";
     if (items > 1 && split) {
         os << indent << "if (w0 + " << u64((std::uint64_t)(items - 1) * tpb) << " < " << u64(total) << ") {\n"
            << indent << "    #pragma unroll\n" << indent << "    for (int j = 0; j < " << items << "; ++j) {\n"
            << indent << "        const unsigned long long w = w0 + (unsigned long long)j * " << tpb << "ull;\n"
-           << indent << "        symgbBody" << k << "<" << l2 << ">(x, xw, p, c, res, dp, w / " << S
+           << indent << "        symgbBody" << k << targs << "(x, xw, p, c, res, dp, w / " << S
            << "ull, (unsigned)(w % " << S << "ull));\n"
            << indent << "    }\n" << indent << "} else {\n";
     }
     if (items > 1) os << indent << "#pragma unroll\n" << indent << "for (int j = 0; j < " << items << "; ++j) {\n";
     else os << indent << "{\n" << indent << "    const int j = 0;\n";
     os << indent << "    const unsigned long long w = w0 + (unsigned long long)j * " << tpb << "ull;\n"
-       << indent << "    if (w < " << u64(total) << ") symgbBody" << k << "<" << l2 << ">(x, xw, p, c, res, dp, w / "
+       << indent << "    if (w < " << u64(total) << ") symgbBody" << k << targs << "(x, xw, p, c, res, dp, w / "
        << S << "ull, (unsigned)(w % " << S << "ull));\n"
        << indent << "}\n";
     if (items > 1 && split) os << indent << "}\n";
@@ -281,24 +292,24 @@ void emitGroups(std::ostringstream& os, int k, const symgb_kernel_desc& d, unsig
 
 // The work of kernel k in either item layout.
 void emitWork(std::ostringstream& os, int k, const symgb_kernel_desc& d, std::size_t ops, unsigned S, int tpb,
-              int items, int l2, const std::string& b0, const char* indent, bool grouped) {
+              int items, int l2, const std::string& b0, const char* indent, bool grouped, int order = 0) {
     const bool split = ops * (std::size_t)items <= kSplitOps;
     if (grouped) emitGroups(os, k, d, S, tpb, items, l2, b0, indent, split);
-    else emitItems(os, k, d.num_instances * S, S, tpb, items, l2, b0, indent, split);
+    else emitItems(os, k, d.num_instances * S, S, tpb, items, l2, b0, indent, split, order);
 }
 
 // Dispatch of block `b` over the kernels of one launch (kernel-major block
 // ranges, each kernel's work items in consecutive blocks).
 void emitDispatch(std::ostringstream& os, const std::vector<int>& ks, const std::vector<symgb_kernel_desc>& descs,
                   const std::vector<std::size_t>& opCount, unsigned S, int tpb, int items, int l2, const char* indent,
-                  bool grouped) {
+                  bool grouped, int order = 0) {
     std::uint64_t first = 0;
     const std::string inner = std::string(indent) + "    ";
     for (std::size_t q = 0; q < ks.size(); ++q) {
         const int k = ks[q];
         const std::uint64_t blocks = kernelBlocks(descs[k], S, tpb, items, grouped);
         os << indent << (q ? "else " : "") << "if (b < " << u64(first + blocks) << ") {\n";
-        emitWork(os, k, descs[k], opCount[k], S, tpb, items, l2, "b - " + u64(first), inner.c_str(), grouped);
+        emitWork(os, k, descs[k], opCount[k], S, tpb, items, l2, "b - " + u64(first), inner.c_str(), grouped, order);
         os << indent << "}\n";
         first += blocks;
     }
@@ -329,6 +340,35 @@ std::string launchBounds(int tpb, int minBlocks) {
     const int fit = std::min(minBlocks, 2048 / std::max(1, tpb));
     if (fit > 0) s += ", " + std::to_string(fit);
     return s + ")";
+}
+
+// How a launch stands to the one before it (programmatic dependent launch).
+// A launch of another dependency level than its predecessor's waits for it
+// before its first read of x.  Launches of one level read nothing of each
+// other's: they let the next one in at once and run side by side, each waiting
+// at its end instead, so that a launch is complete only when all before it
+// are and the next level's wait covers the whole level.  Cloth 64 x 64, one
+// set (18 kernels, 17 of them of one level, 12 to 9000 instances each): 75.6 us
+// one after another, 58.8 so, of which 47 are the host's launches; 100 x 100, 64
+// sets: 2.10 -> 2.03 ms.
+struct LaunchOrder {
+    bool waitFirst;  // before the first read of x
+    bool letInFirst;  // the next launch may start beside this one
+};
+
+// Prologue of a launch.  One work item per thread (strided): the wait goes
+// behind the table loads of the body, which nothing writes (template argument
+// `order`), and the tables arrive while the predecessor drains.
+int emitPrologue(std::ostringstream& os, const LaunchOrder& o, bool inBody) {
+    const int order = (o.waitFirst ? 1 : 0) | (o.letInFirst ? 2 : 0);
+    if (inBody) return order;
+    if (order) os << "    x = symgbOrder<" << order << ">(x);\n";
+    return 0;
+}
+
+void emitEpilogue(std::ostringstream& os, const LaunchOrder& o) {
+    if (!o.letInFirst) os << "    symgbLaunchDependents();\n";
+    if (!o.waitFirst) os << "    symgbDependencyWait();\n";
 }
 
 }  // namespace
@@ -410,21 +450,26 @@ JitSource generateModule(const std::vector<symgb_kernel_desc>& descs, int numLev
         if (descs[k].num_instances) byLevel[L].push_back((int)k);
     }
     if (cfg.kind == JIT_PLAIN) {
-        for (std::size_t k = 0; k < descs.size(); ++k) {
-            const std::uint64_t total = descs[k].num_instances * S;
-            if (!total) continue;
+        std::vector<int> ks;
+        for (std::size_t k = 0; k < descs.size(); ++k)
+            if (descs[k].num_instances * S) ks.push_back((int)k);
+        for (std::size_t q = 0; q < ks.size(); ++q) {
+            const int k = ks[q], level = descs[k].level;
             const int tpb = cfg.kernelTpb.at(k);
             const int items = checkedItems(cfg.kernelItems.at(k));
             const std::string name = "symgb_k" + std::to_string(k);
-            os << "extern \"C\" __global__ void " << launchBounds(tpb, cfg.minBlocks) << " " << name << params << ") {\n"
-               << "    symgbDependencyWait();\n    symgbLaunchDependents();\n";
-            emitWork(os, (int)k, descs[k], opCount[k], S, tpb, items, 0, "(unsigned long long)blockIdx.x", "    ",
-                     grouped);
+            const LaunchOrder o{q == 0 || descs[ks[q - 1]].level != level,
+                                q + 1 < ks.size() && descs[ks[q + 1]].level == level};
+            os << "extern \"C\" __global__ void " << launchBounds(tpb, cfg.minBlocks) << " " << name << params << ") {\n";
+            const int order = emitPrologue(os, o, items == 1 && !grouped);
+            emitWork(os, k, descs[k], opCount[k], S, tpb, items, 0, "(unsigned long long)blockIdx.x", "    ", grouped,
+                     order);
+            emitEpilogue(os, o);
             os << "}\n\n";
-            out.launches.push_back({name, (int)k, -1, kernelBlocks(descs[k], S, tpb, items, grouped), tpb, items,
-                                    false});
+            out.launches.push_back({name, k, -1, kernelBlocks(descs[k], S, tpb, items, grouped), tpb, items, false});
         }
     } else if (cfg.kind == JIT_LEVELS) {
+        const LaunchOrder o{true, false};
         for (int L = 0; L < numLevels; ++L) {
             std::vector<int> ks = byLevel[L];
             if (ks.empty()) continue;
@@ -434,10 +479,11 @@ JitSource generateModule(const std::vector<symgb_kernel_desc>& descs, int numLev
             const int tpb = cfg.levelTpb.at(L);
             const int items = checkedItems(cfg.levelItems.at(L));
             const std::string name = "symgb_l" + std::to_string(L);
-            os << "extern \"C\" __global__ void " << launchBounds(tpb, cfg.minBlocks) << " " << name << params << ") {\n"
-               << "    symgbDependencyWait();\n    symgbLaunchDependents();\n"
-               << "    const unsigned long long b = blockIdx.x;\n";
-            emitDispatch(os, ks, descs, opCount, S, tpb, items, 0, "    ", grouped);
+            os << "extern \"C\" __global__ void " << launchBounds(tpb, cfg.minBlocks) << " " << name << params << ") {\n";
+            const int order = emitPrologue(os, o, items == 1 && !grouped);
+            os << "    const unsigned long long b = blockIdx.x;\n";
+            emitDispatch(os, ks, descs, opCount, S, tpb, items, 0, "    ", grouped, order);
+            emitEpilogue(os, o);
             os << "}\n\n";
             out.launches.push_back({name, -1, L, blocksOf(ks, descs, S, tpb, items, grouped), tpb, items, false});
         }

@@ -128,6 +128,15 @@ __device__ bool symgbGridBarrier(B* bar, int* hostError, unsigned long long time
 // running; it waits here until that kernel has finished and its writes are
 // visible.  Without the launch attribute the wait returns at once.  The
 // trigger lets the next such kernel be scheduled as soon as every block of
-// this one has started (it still waits for this one to finish).
+// this one has issued it or ended.
 __device__ __forceinline__ void symgbDependencyWait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void symgbLaunchDependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// ORDER & 1: wait, with x passing through the wait so that no read of x can
+// move above it; ORDER & 2: let the next kernel in.
+#define SYMGB_ORDERED
+template <int ORDER>
+__device__ __forceinline__ const double* symgbOrder(const double* x) {
+    if (ORDER & 1) asm volatile("griddepcontrol.wait;" : "+l"(x) : : "memory");
+    if (ORDER & 2) symgbLaunchDependents();
+    return x;
+}
