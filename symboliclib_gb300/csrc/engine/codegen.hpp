@@ -78,6 +78,7 @@ struct JitModule {
     std::vector<JitLaunch> launches;
     std::vector<const void*> kernels;
     std::vector<int> registers;  // per launch: registers per thread of the compiled kernel
+    std::vector<int> blocksPerSm;  // cooperative launches: most resident blocks of an SM
     double compileSeconds = 0;
     bool grouped = false;        // launch with the padded tables (GroupedTables)
     bool direct = false;         // writes some results straight into res

@@ -469,10 +469,11 @@ __global__ void __maxnreg__(EvalRegs<ITEMS>::value) evalKernel(EvalArgs A) {
 __global__ void gatherKernel(const double* __restrict__ x, const std::uint32_t* __restrict__ ids, std::uint64_t len,
                              unsigned S, double* __restrict__ out) {
     const std::uint64_t w = (std::uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const double* xr = symgbOrder<1>(x);
     if (w >= len * S) return;
     const std::uint64_t s = S == 1 ? 0 : w / len;
     const std::uint64_t j = w - s * len;
-    out[w] = __ldg(x + (std::uint64_t)__ldg(ids + j) * S + s);
+    out[w] = __ldg(xr + (std::uint64_t)__ldg(ids + j) * S + s);
 }
 
 }  // namespace

@@ -57,14 +57,46 @@ namespace {
 
 // ------------------------------------------------------------------ device side
 
+// The copies between a caller's buffers and x or res below are launched with
+// programmatic stream serialisation, as the run's own launches are (chained):
+// each waits for its predecessor before it touches memory and lets the next
+// one in when it is done.  A boundary between two such kernels costs about 1 us
+// of the stream; one with a copy operation or without the attribute 2 to 4 (cotan
+// 100 x 100, inputs and results on the device: 18.4 us with copy operations and an
+// unchained first launch, 12.2 so).
+
+// dst[q] = src[q]; 16 bytes at a time where both are aligned to it.
+__global__ void __launch_bounds__(256) copyKernel(const double* src, double* dst, std::uint64_t n) {
+    constexpr unsigned kPer = 4;
+    src = symgbOrder<1>(src);
+    const std::uint64_t t = (std::uint64_t)blockIdx.x * 256 * kPer + threadIdx.x;
+    if ((((std::uintptr_t)src | (std::uintptr_t)dst) & 15) == 0) {
+        const double2* s2 = reinterpret_cast<const double2*>(src);
+        double2* d2 = reinterpret_cast<double2*>(dst);
+#pragma unroll
+        for (unsigned k = 0; k < kPer; ++k)
+            if (t + k * 256 < n / 2) d2[t + k * 256] = s2[t + k * 256];
+        if ((n & 1) && t == 0) dst[n - 1] = src[n - 1];
+    } else {
+#pragma unroll
+        for (unsigned k = 0; k < 2 * kPer; ++k) {
+            const std::uint64_t q = (std::uint64_t)blockIdx.x * 512 * kPer + threadIdx.x + k * 256;
+            if (q < n) dst[q] = src[q];
+        }
+    }
+    symgbLaunchDependents();
+}
+
 // x[(start + j) * S + s] = in[s * len + j]
 __global__ void scatterKernel(const double* __restrict__ in, std::uint64_t start, std::uint64_t len, unsigned S,
                               double* __restrict__ x) {
     const std::uint64_t w = (std::uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    in = symgbOrder<1>(in);
     if (w >= len * S) return;
     const std::uint64_t j = w / S;
     const unsigned s = (unsigned)(w - j * S);
     x[(start + j) * S + s] = __ldg(in + (std::uint64_t)s * len + j);
+    symgbLaunchDependents();
 }
 
 // The same two copies for many value sets, through a 32 x 32 tile in shared
@@ -83,6 +115,7 @@ __global__ void __launch_bounds__(256) gatherSetsKernel(const double* __restrict
     const std::uint64_t j0 = (std::uint64_t)blockIdx.x * kSetTile;
     const unsigned s0 = blockIdx.y * kSetTile;
     const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    x = symgbOrder<1>(x);
     for (unsigned p = warp; p < kSetTile; p += 8) {
         const std::uint64_t j = j0 + p;
         if (j < len && s0 + lane < S) tile[p][lane] = __ldg(x + (std::uint64_t)__ldg(ids + j) * S + s0 + lane);
@@ -92,6 +125,7 @@ __global__ void __launch_bounds__(256) gatherSetsKernel(const double* __restrict
         const std::uint64_t j = j0 + lane;
         if (s0 + q < S && j < len) out[(std::uint64_t)(s0 + q) * len + j] = tile[lane][q];
     }
+    symgbLaunchDependents();
 }
 
 // x[(start + j) * S + s] = in[s * len + j]
@@ -101,6 +135,7 @@ __global__ void __launch_bounds__(256) scatterSetsKernel(const double* __restric
     const std::uint64_t j0 = (std::uint64_t)blockIdx.x * kSetTile;
     const unsigned s0 = blockIdx.y * kSetTile;
     const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    in = symgbOrder<1>(in);
     for (unsigned q = warp; q < kSetTile; q += 8) {
         const std::uint64_t j = j0 + lane;
         if (s0 + q < S && j < len) tile[lane][q] = __ldg(in + (std::uint64_t)(s0 + q) * len + j);
@@ -110,6 +145,7 @@ __global__ void __launch_bounds__(256) scatterSetsKernel(const double* __restric
         const std::uint64_t j = j0 + p;
         if (j < len && s0 + lane < S) x[(start + j) * S + s0 + lane] = tile[p][lane];
     }
+    symgbLaunchDependents();
 }
 
 // Padded copy of one kernel's table rows for the compiled executor's grouped
@@ -129,13 +165,54 @@ __global__ void padRowsKernel(const T* __restrict__ src, T* __restrict__ dst, st
 __global__ void restGatherKernel(const double* __restrict__ x, const std::uint32_t* __restrict__ pos,
                                  const std::uint32_t* __restrict__ slot, std::uint64_t count, double* __restrict__ res) {
     const std::uint64_t t = (std::uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    x = symgbOrder<1>(x);
     if (t < count) res[__ldg(pos + t)] = __ldg(x + __ldg(slot + t));
+    symgbLaunchDependents();
 }
 
 // Value-set counts from which the tiled kernels are used.
 constexpr unsigned kTiledSets = 8;
 
 // ------------------------------------------------------------------ host side
+
+// Whether a launch on the unit's stream may overlap its start with what is
+// before it.  Not inside a capture of the caller's, whose dependencies may be
+// of any kind.
+bool chained(const symgb_unit* u) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(u->stream, &status) == cudaSuccess) return status == cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return false;
+}
+
+template <class... P, class... A>
+cudaError_t launchChained(const symgb_unit* u, void (*fn)(P...), dim3 grid, A... args) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(256);
+    cfg.stream = u->stream;
+    cfg.attrs = at;
+    cfg.numAttrs = chained(u) ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, fn, static_cast<P>(args)...);
+}
+
+cudaError_t copyChained(const symgb_unit* u, const double* src, double* dst, std::uint64_t n) {
+    return n ? launchChained(u, copyKernel, dim3((unsigned)((n + 2047) / 2048)), src, dst, n) : cudaSuccess;
+}
+
+// Memory of the unit's device, for the copy kernel; other memory takes the
+// runtime's copies.
+bool onDevice(const symgb_unit* u, const void* p) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeDevice && a.device == u->device;
+}
 
 }  // namespace
 
@@ -379,12 +456,19 @@ int getModule(symgb_unit* u, int kind, std::shared_ptr<const JitModule>* out, do
 // Enqueues one evaluation with the compiled executor.  Launches after the
 // first overlap their start-up with the previous launch (programmatic
 // dependent launch; a level's first kernel waits for its predecessor before
-// reading x, the level's others run beside it).
+// reading x, the level's others run beside it); with `chainFirst` the first
+// launch's too with whatever is before it on the stream.
 // With `kernelEvents`, runs the plain module without that overlap and
 // records an event before and after each kernel's launch.
-int enqueueCompiled(symgb_unit* u, const std::vector<cudaEvent_t>* kernelEvents) {
+int enqueueCompiled(symgb_unit* u, const std::vector<cudaEvent_t>* kernelEvents, bool chainFirst) {
     std::shared_ptr<const JitModule> m;
-    if (int e = getModule(u, kernelEvents ? SYMGB_SCHEDULE_PLAIN : u->sched.kind, &m)) return e;
+    if (kernelEvents) {
+        if (int e = getModule(u, SYMGB_SCHEDULE_PLAIN, &m)) return e;
+    } else {
+        if (!u->current)
+            if (int e = getModule(u, u->sched.kind, &u->current)) return e;
+        m = u->current;
+    }
     const double* x = u->x.ptr;
     double* xw = u->x.ptr;
     const std::uint32_t* p = m->grouped ? u->p4.ptr : u->p.ptr;
@@ -405,8 +489,7 @@ int enqueueCompiled(symgb_unit* u, const std::vector<cudaEvent_t>* kernelEvents)
         unsigned na = 0;
         unsigned grid = (unsigned)L.blocks;
         if (L.cooperative) {
-            int perSm = 0;
-            SYMGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, m->kernels[j], L.tpb, 0));
+            int perSm = m->blocksPerSm[j];
             if (perSm < 1) return fail(SYMGB_ERR_ARGUMENT, "persistent schedule: kernel does not fit on an SM");
             if (u->sched.blocks_per_sm > 0) perSm = std::min(perSm, u->sched.blocks_per_sm);
             grid = std::max(1u, std::min<unsigned>(grid, (unsigned)(perSm * u->smCount)));
@@ -414,7 +497,7 @@ int enqueueCompiled(symgb_unit* u, const std::vector<cudaEvent_t>* kernelEvents)
             at[na].val.cooperative = 1;
             ++na;
         }
-        if (j > 0 && !kernelEvents) {
+        if (j > 0 ? !kernelEvents : chainFirst && !L.cooperative) {
             at[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
             at[na].val.programmaticStreamSerializationAllowed = 1;
             ++na;
@@ -439,8 +522,8 @@ int enqueueCompiled(symgb_unit* u, const std::vector<cudaEvent_t>* kernelEvents)
 // Enqueues one evaluation on the unit's stream.  With `kernelEvents`, runs the
 // plain schedule whatever the unit's and records an event before and after
 // each kernel's launch (per-kernel timing).
-int enqueueRun(symgb_unit* u, const std::vector<cudaEvent_t>* kernelEvents = nullptr) {
-    if (u->compiledExec()) return enqueueCompiled(u, kernelEvents);
+int enqueueRun(symgb_unit* u, const std::vector<cudaEvent_t>* kernelEvents = nullptr, bool chainFirst = false) {
+    if (u->compiledExec()) return enqueueCompiled(u, kernelEvents, chainFirst);
     u->lastRunDirect = false;
     if (int e = buildTiles(u)) return e;
     const int items = u->items();
@@ -567,10 +650,25 @@ int runAsync(symgb_unit* u) {
     if (!u->initialized) return fail(SYMGB_ERR_STATE, "run before init");
     // A run that writes its results straight into res waits (on the unit's
     // stream) for the asynchronous copies still reading the previous ones.
+    bool chain = chained(u);
+    const bool capturing = !chain;
     if (u->compiledExec() && u->directOutputs && u->directRows && u->numSets == 1)
         for (cudaEvent_t e : u->copyDone)
-            if (e) SYMGB_CUDA(cudaStreamWaitEvent(u->stream, e, 0));
-    if (u->sched.use_graph) {
+            if (e) {
+                SYMGB_CUDA(cudaStreamWaitEvent(u->stream, e, 0));
+                chain = false;
+            }
+    // A run of many launches is replayed as a graph from its second time on
+    // (use_graph: from the first).  A chained launch costs the host 1.4 us and
+    // the stream no more, a graph of any size the host 1 us and the stream 2 at
+    // either end: 3 launches between two copies take 6.5 us launch by launch and
+    // 8.3 as a graph, 8 take 13.4 and 12.4, 18 take 26.3 and 20.6.  The first run
+    // of a configuration goes launch by launch, so a configuration that runs
+    // once does not pay for a graph; nor is one made inside a capture of the
+    // caller's, which takes the launches themselves.
+    constexpr int kGraphLaunches = 6;
+    const bool graph = u->sched.use_graph || (u->ranBefore && u->launchesPerRun >= kGraphLaunches && !capturing);
+    if (graph) {
         if (!u->graphValid) {
             if (u->compiledExec()) {  // nothing may be compiled or loaded during the capture
                 std::shared_ptr<const JitModule> m;
@@ -579,21 +677,32 @@ int runAsync(symgb_unit* u) {
             if (int e = buildTiles(u)) return e;
             // smem attributes must be set outside capture
             cudaGraph_t g;
-            SYMGB_CUDA(cudaStreamBeginCapture(u->stream, cudaStreamCaptureModeThreadLocal));
-            int e = enqueueRun(u);
-            cudaError_t ce = cudaStreamEndCapture(u->stream, &g);
+            cudaStream_t saved = u->stream;
+            u->stream = u->ownStream;  // a stream of the caller's may be one that cannot be captured
+            cudaError_t ce = cudaStreamBeginCapture(u->stream, cudaStreamCaptureModeThreadLocal);
+            int e = SYMGB_OK;
+            if (ce == cudaSuccess) {
+                e = enqueueRun(u);
+                ce = cudaStreamEndCapture(u->stream, &g);
+            }
+            u->stream = saved;
             if (e) return e;
             if (ce != cudaSuccess) return fail(SYMGB_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(ce));
-            SYMGB_CUDA(cudaGraphInstantiate(&u->graph, g, 0));
+            ce = cudaGraphInstantiate(&u->graph, g, 0);
             cudaGraphDestroy(g);
+            if (ce != cudaSuccess)
+                return fail(SYMGB_ERR_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(ce));
             u->graphValid = true;
+            u->graphDirect = u->lastRunDirect;
         }
         SYMGB_CUDA(cudaGraphLaunch(u->graph, u->stream));
+        u->lastRunDirect = u->graphDirect;
         u->lastLaunches = u->launchesPerRun;
         return SYMGB_OK;
     }
-    int e = enqueueRun(u);
+    int e = enqueueRun(u, nullptr, chain);
     u->lastLaunches = u->launchesPerRun;
+    u->ranBefore = e == SYMGB_OK;
     return e;
 }
 
@@ -813,9 +922,8 @@ static bool resultsInRes(symgb_unit* u, int* err) {
     *err = SYMGB_OK;
     if (!u->lastRunDirect || u->numSets != 1) return false;
     if (u->restCount) {
-        restGatherKernel<<<(unsigned)((u->restCount + 255) / 256), 256, 0, u->stream>>>(
-            u->x.ptr, u->restPos.ptr, u->restSlot.ptr, u->restCount, u->res.ptr);
-        const cudaError_t e = cudaGetLastError();
+        const cudaError_t e = launchChained(u, restGatherKernel, dim3((unsigned)((u->restCount + 255) / 256)), u->x.ptr,
+                                            u->restPos.ptr, u->restSlot.ptr, u->restCount, u->res.ptr);
         if (e != cudaSuccess) *err = fail(SYMGB_ERR_CUDA, std::string("rest gather: ") + cudaGetErrorString(e));
     }
     return true;
@@ -827,7 +935,9 @@ int symgb_get_result_sets_device(symgb_unit_t u, double* d, int k) {
     int err = SYMGB_OK;
     if (resultsInRes(u, &err)) {
         if (err) return err;
-        if (u->outLength[k])
+        if (onDevice(u, d))
+            SYMGB_CUDA(copyChained(u, u->res.ptr + u->outStart[k], d, u->outLength[k]));
+        else if (u->outLength[k])
             SYMGB_CUDA(cudaMemcpyAsync(d, u->res.ptr + u->outStart[k], u->outLength[k] * 8, cudaMemcpyDefault,
                                        u->stream));
         return SYMGB_OK;
@@ -836,12 +946,10 @@ int symgb_get_result_sets_device(symgb_unit_t u, double* d, int k) {
     const std::uint64_t work = len * u->numSets;
     if (work && u->numSets >= kTiledSets) {
         const dim3 grid((unsigned)((len + kSetTile - 1) / kSetTile), (unsigned)((u->numSets + kSetTile - 1) / kSetTile));
-        gatherSetsKernel<<<grid, 256, 0, u->stream>>>(u->x.ptr, u->ids.ptr + u->outStart[k], len, (unsigned)u->numSets, d);
-        SYMGB_CUDA(cudaGetLastError());
+        SYMGB_CUDA(launchChained(u, gatherSetsKernel, grid, u->x.ptr, u->ids.ptr + u->outStart[k], len, u->numSets, d));
     } else if (work) {
-        gatherKernel<<<(unsigned)((work + 255) / 256), 256, 0, u->stream>>>(u->x.ptr, u->ids.ptr + u->outStart[k], len,
-                                                                            (unsigned)u->numSets, d);
-        SYMGB_CUDA(cudaGetLastError());
+        SYMGB_CUDA(launchChained(u, gatherKernel, dim3((unsigned)((work + 255) / 256)), u->x.ptr,
+                                 u->ids.ptr + u->outStart[k], len, u->numSets, d));
     }
     return SYMGB_OK;
 }
@@ -884,25 +992,31 @@ int symgb_get_result_sets(symgb_unit_t u, double* d, int k) {
 
 int symgb_get_result(symgb_unit_t u, double* d, int k) { return symgb_get_result_sets(u, d, k); }
 
+// Input container i of all value sets from `d` [set][j] into x [slot][set].
+static int scatterArg(symgb_unit* u, const double* d, int i) {
+    const std::uint64_t len = u->argLength[i], work = len * u->numSets;
+    if (work && u->numSets >= kTiledSets) {
+        const dim3 grid((unsigned)((len + kSetTile - 1) / kSetTile), (unsigned)((u->numSets + kSetTile - 1) / kSetTile));
+        SYMGB_CUDA(launchChained(u, scatterSetsKernel, grid, d, u->argStart[i], len, u->numSets, u->x.ptr));
+    } else if (work) {
+        SYMGB_CUDA(launchChained(u, scatterKernel, dim3((unsigned)((work + 255) / 256)), d, u->argStart[i], len,
+                                 u->numSets, u->x.ptr));
+    }
+    return SYMGB_OK;
+}
+
 int symgb_set_arg_sets_device(symgb_unit_t u, const double* d, int i) {
     if (!u || !u->initialized) return fail(SYMGB_ERR_STATE, "set_arg before init");
     if (i < 0 || (std::size_t)i >= u->argStart.size() || !d) return fail(SYMGB_ERR_ARGUMENT, "bad argument index");
     const std::uint64_t len = u->argLength[i];
     if (u->numSets == 1) {
-        SYMGB_CUDA(cudaMemcpyAsync(u->x.ptr + u->argStart[i], d, len * 8, cudaMemcpyDeviceToDevice, u->stream));
+        if (onDevice(u, d))
+            SYMGB_CUDA(copyChained(u, d, u->x.ptr + u->argStart[i], len));
+        else
+            SYMGB_CUDA(cudaMemcpyAsync(u->x.ptr + u->argStart[i], d, len * 8, cudaMemcpyDeviceToDevice, u->stream));
         return SYMGB_OK;
     }
-    const std::uint64_t work = len * u->numSets;
-    if (work && u->numSets >= kTiledSets) {
-        const dim3 grid((unsigned)((len + kSetTile - 1) / kSetTile), (unsigned)((u->numSets + kSetTile - 1) / kSetTile));
-        scatterSetsKernel<<<grid, 256, 0, u->stream>>>(d, u->argStart[i], len, (unsigned)u->numSets, u->x.ptr);
-        SYMGB_CUDA(cudaGetLastError());
-    } else if (work) {
-        scatterKernel<<<(unsigned)((work + 255) / 256), 256, 0, u->stream>>>(d, u->argStart[i], len, (unsigned)u->numSets,
-                                                                             u->x.ptr);
-        SYMGB_CUDA(cudaGetLastError());
-    }
-    return SYMGB_OK;
+    return scatterArg(u, d, i);
 }
 
 int symgb_set_arg_sets(symgb_unit_t u, const double* d, int i) {
@@ -1164,6 +1278,7 @@ int symgb_time_kernels(symgb_unit_t u, int reps, void* flush, uint64_t flush_byt
         u->timingEvents.push_back(ev);
     }
     for (std::size_t k = 0; k < nk; ++k) us_per_kernel[k] = 0.0;
+    const int launchesPerRun = u->launchesPerRun;  // of the unit's own schedule
     for (int r = 0; r < reps; ++r) {
         if (flush && flush_bytes) SYMGB_CUDA(cudaMemsetAsync(flush, r & 0xff, flush_bytes, u->stream));
         const std::vector<cudaEvent_t> evs(u->timingEvents.begin() + per * r, u->timingEvents.begin() + per * (r + 1));
@@ -1175,6 +1290,7 @@ int symgb_time_kernels(symgb_unit_t u, int reps, void* flush, uint64_t flush_byt
             }
         if (int e = enqueueRun(u, &evs)) return e;
     }
+    u->launchesPerRun = launchesPerRun;
     SYMGB_CUDA(cudaStreamSynchronize(u->stream));
     for (int r = 0; r < reps; ++r)
         for (std::size_t k = 0; k < nk; ++k) {
@@ -1209,8 +1325,7 @@ int symgb_num_sets(symgb_unit_t u) { return u ? u->numSets : 0; }
 
 int symgb_set_stream(symgb_unit_t u, void* stream) {
     if (!u || !u->initialized) return fail(SYMGB_ERR_STATE, "set_stream before init");
-    u->stream = stream ? (cudaStream_t)stream : u->ownStream;
-    u->dropGraph();
+    u->stream = stream ? (cudaStream_t)stream : u->ownStream;  // a graph runs on whichever
     return SYMGB_OK;
 }
 

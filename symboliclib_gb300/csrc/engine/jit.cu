@@ -142,6 +142,16 @@ int loadModule(const JitSource& src, std::shared_ptr<const JitModule>* out, std:
         }
         m->kernels.push_back((const void*)k);
         m->registers.push_back(fa.numRegs);
+        int perSm = 0;
+        if (L.cooperative) {
+            ce = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, (const void*)k, L.tpb, 0);
+            if (ce != cudaSuccess) {
+                *err = "cudaOccupancyMaxActiveBlocksPerMultiprocessor(" + L.name + "): " + cudaGetErrorString(ce);
+                cudaLibraryUnload(e.library);
+                return SYMGB_ERR_CUDA;
+            }
+        }
+        m->blocksPerSm.push_back(perSm);
     }
     m->compileSeconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     e.module = m;

@@ -127,13 +127,16 @@ struct symgb_unit {
     std::map<std::array<std::uint32_t, 6>, std::uint32_t> stagingCache;
     std::size_t tilesFor = 0;  // configuration the tile table was built for
     int tilesSets = -1, tilesItems = -1, tilesMath = -1;
+    // One run as a graph (runAsync), until the configuration changes:
+    // graphDirect is lastRunDirect after it, ranBefore whether the configuration
+    // has run launch by launch.
     cudaGraphExec_t graph = nullptr;
-    bool graphValid = false;
+    bool graphValid = false, graphDirect = false, ranBefore = false;
     // Compiled executor: modules by configuration key (schedule kind, math,
-    // value sets, block sizes); `jit` is the current schedule's.
+    // value sets, block sizes); `current` is the current configuration's, once
+    // it has been looked up.
     std::map<std::string, std::shared_ptr<const symgb::engine::JitModule>> jitModules;
-    std::shared_ptr<const symgb::engine::JitModule> jit;
-    std::string jitKey;
+    std::shared_ptr<const symgb::engine::JitModule> current;
     int lastLaunches = 0;
     int launchesPerRun = 0;
     unsigned long long barrierTimeoutNs = 2000000000ull;
@@ -141,10 +144,13 @@ struct symgb_unit {
 
     ~symgb_unit() { release(); }
 
+    // Forgets what was made for the current configuration (a graph in flight is
+    // freed when it completes).
     void dropGraph() {
         if (graph) cudaGraphExecDestroy(graph);
         graph = nullptr;
-        graphValid = false;
+        graphValid = ranBefore = false;
+        current.reset();
     }
 
     void release() {
