@@ -22,6 +22,8 @@
 
 #include <algorithm>
 #include <cstdio>
+#include <map>
+#include <set>
 #include <cstring>
 #include <sstream>
 #include <stdexcept>
@@ -70,27 +72,85 @@ const char* libName(int op) {
 // res[dp[start + i]] (their final positions) instead of x.  L2 = 1 reads x
 // through L2 only (values written earlier in the same launch, persistent
 // schedule).  Returns the number of operations of the template.
+//   With intMuls > 0: symgbMixed<k>, the strided body with that many of its
+//     products, evenly spread, and the first products of its divisions and
+//     square roots on the integer pipes (prelude: symgbMulInt), the same bits
+//     as symgbBody<k>'s.  It returns whether an operand was outside what those
+//     cover; the caller then evaluates symgbBody<k>, which stores the same
+//     results again.  A product's range is checked at its factors that come
+//     from loads or FP64 instructions, once each; products of up to four of
+//     them need no check.
+// `called`: emitted as a function of its own instead of into its callers.
 std::size_t emitBody(std::ostringstream& os, int k, const symgb_kernel_desc& d, int math, unsigned S,
-                     const GroupedTables* grouped, const std::vector<std::int64_t>* direct) {
+                     const GroupedTables* grouped, const std::vector<std::int64_t>* direct, bool called,
+                     int intMuls = 0) {
     std::vector<std::uint64_t> loads;
     const std::vector<LinOp> ops = linearCode(d, math, &loads);
     const std::uint64_t n = d.num_instances;
     const bool g = grouped != nullptr;
     const char* in = g ? "        " : "    ";
-    os << "// kernel " << k << ": " << n << " instances, level " << d.level << ", " << loads.size() << " loads, "
+    const bool mixed = intMuls > 0;
+    if (!mixed) os << "// kernel " << k << ": " << n << " instances, level " << d.level << ", " << loads.size() << " loads, "
        << ops.size() << " operations\n";
+    if (called && !mixed) os << "#ifndef SYMGB_CALLED\n#define SYMGB_CALLED\n#endif\n";
     if (g)
         os << "template <int L2, int IT, bool FULL>\n__device__ __forceinline__ void symgbGroup" << k
            << "(const double* SYMGB_XR x, double* SYMGB_XR xw, const unsigned* __restrict__ p, "
               "const double* __restrict__ c, double* __restrict__ res, const unsigned* __restrict__ dp, "
               "unsigned long long g, unsigned s) {\n";
     else
-        os << "template <int L2, int ORDER = 0>\n__device__ __forceinline__ void symgbBody" << k
+        os << "template <int L2, int ORDER = 0>\n__device__ " << (called ? "SYMGB_CALLED " : "__forceinline__ ")
+           << (mixed ? "bool symgbMixed" : "void symgbBody") << k
            << "(const double* SYMGB_XR x, double* SYMGB_XR xw, const unsigned* __restrict__ p, "
               "const double* __restrict__ c, double* __restrict__ res, const unsigned* __restrict__ dp, "
               "unsigned long long i, unsigned s) {\n";
     std::vector<std::string> cur(256);
     int next = 0;
+    // Integer products (mixed bodies): literals, factors of a value, values
+    // whose range has been checked, values whose significand is at hand.
+    std::map<std::string, std::uint64_t> literals;
+    std::map<std::string, int> factors;
+    std::set<std::string> checked, split;
+    int mulsSeen = 0, mulsTaken = 0, mulCount = 0;
+    for (const LinOp& L : ops) mulCount += L.op == OP_MUL;
+    if (mixed) os << "    bool outside = false;\n";
+    auto inWindow = [](std::uint64_t b) {
+        const unsigned e = (unsigned)(b >> 52) & 0x7ffu;
+        return e >= 768 && e < 1279;
+    };
+    auto check = [&](const std::string& v) {  // v's range, at run time: one factor from here on
+        if (checked.insert(v).second && !literals.count(v)) os << in << "outside |= symgbOutside(" << v << ");\n";
+        factors[v] = 1;
+    };
+    auto sig = [&](const std::string& v) {
+        if (split.insert(v).second) os << in << "const unsigned s" << v << " = symgbSig(" << v << ");\n";
+        return "s" + v;
+    };
+    // a * b on the integer pipes, or nothing where they do not cover it.
+    auto intProduct = [&](std::string a, std::string b) -> std::string {
+        if (literals.count(a)) std::swap(a, b);
+        if (literals.count(a)) return std::string();
+        const auto lit = literals.find(b);
+        if (lit != literals.end()) {
+            if (!inWindow(lit->second)) return std::string();
+            const int K = (int)((lit->second >> 52) & 0x7ff) - 1023;
+            if (!(lit->second & 0xfffffffffffffull) && K >= -64 && K <= 64) {
+                if (!factors.count(a) || factors[a] > 3) check(a);
+                factors["="] = factors[a] + 1;
+                return "symgbMulPow2<" + std::to_string(K) + ", " + std::to_string((int)(lit->second >> 63)) + ">(" + a + ")";
+            }
+            factors[b] = 1;
+        }
+        if ((long long)mulsSeen * intMuls / std::max(1, mulCount) < mulsTaken) return std::string();
+        if (!factors.count(a)) check(a);
+        if (!factors.count(b)) check(b);
+        if (factors[a] + factors[b] > 4) check(factors[a] > factors[b] ? a : b);
+        if (factors[a] + factors[b] > 4) check(factors[a] > factors[b] ? a : b);
+        ++mulsTaken;
+        factors["="] = factors[a] + factors[b];
+        const std::string sa = sig(a), sb = sig(b);
+        return "symgbMulInt(" + a + ", " + b + ", " + sa + ", " + sb + ")";
+    };
     auto fresh = [&](int reg) -> std::string {
         std::string v = "v" + std::to_string(next++);
         if (reg < 0 || reg >= (int)cur.size()) throw std::runtime_error("codegen: register out of range");
@@ -186,13 +246,34 @@ std::size_t emitBody(std::ostringstream& os, int k, const symgb_kernel_desc& d, 
             case OP_LDK: rhs = literal(L.lit); break;
             case OP_ADD: rhs = "__dadd_rn(" + use(L.src[0]) + ", " + use(L.src[1]) + ")"; break;
             case OP_SUB: rhs = "__dsub_rn(" + use(L.src[0]) + ", " + use(L.src[1]) + ")"; break;
-            case OP_MUL: rhs = "__dmul_rn(" + use(L.src[0]) + ", " + use(L.src[1]) + ")"; break;
+            case OP_MUL:
+                if (mixed) {
+                    rhs = intProduct(use(L.src[0]), use(L.src[1]));
+                    ++mulsSeen;
+                    if (!rhs.empty()) break;
+                }
+                rhs = "__dmul_rn(" + use(L.src[0]) + ", " + use(L.src[1]) + ")";
+                break;
             case OP_DIV: rhs = "__ddiv_rn(" + use(L.src[0]) + ", " + use(L.src[1]) + ")"; break;
             case OP_NEG: rhs = "symgbNegate(" + use(L.src[0]) + ")"; break;
             case OP_SQRT: rhs = "__dsqrt_rn(" + use(L.src[0]) + ")"; break;
             case OP_REC: rhs = "__ddiv_rn(1.0, " + use(L.src[0]) + ")"; break;
-            case OP_FDIV: rhs = "symgbFastDiv(" + use(L.src[0]) + ", " + use(L.src[1]) + ")"; break;
-            case OP_FSQRT: rhs = "symgbFastSqrt(" + use(L.src[0]) + ")"; break;
+            case OP_FDIV:
+                if (mixed && !literals.count(use(L.src[0]))) {
+                    const std::string a = use(L.src[0]), b = use(L.src[1]);
+                    if (!factors.count(a) || factors[a] > 1) check(a);  // the division's own range is narrower
+                    rhs = "symgbFastDivInt(" + a + ", " + b + ", " + sig(a) + ", outside)";
+                    break;
+                }
+                rhs = "symgbFastDiv(" + use(L.src[0]) + ", " + use(L.src[1]) + ")"; break;
+            case OP_FSQRT:
+                if (mixed && !literals.count(use(L.src[0]))) {
+                    const std::string a = use(L.src[0]);
+                    if (!factors.count(a) || factors[a] > 3) check(a);
+                    rhs = "symgbFastSqrtInt(" + a + ", " + sig(a) + ", outside)";
+                    break;
+                }
+                rhs = "symgbFastSqrt(" + use(L.src[0]) + ")"; break;
             case OP_FREC: rhs = "symgbFastRec(" + use(L.src[0]) + ")"; break;
             case OP_FMA: rhs = "__fma_rn(" + use(L.src[0]) + ", " + use(L.src[1]) + ", " + use(L.src[2]) + ")"; break;
             case OP_FMS:
@@ -214,10 +295,82 @@ std::size_t emitBody(std::ostringstream& os, int k, const symgb_kernel_desc& d, 
         }
         const std::string v = fresh(L.d);
         os << in << "const double " << v << " = " << rhs << ";\n";
+        if (mixed && L.op == OP_LDK) literals[v] = L.lit;
+        if (mixed && factors.count("=")) {
+            factors[v] = factors["="];
+            factors.erase("=");
+        }
     }
+    if (mixed) os << "    return outside;\n";
     if (g) os << "    }\n";
     os << "}\n\n";
     return ops.size();
+}
+
+// Products of every kernel that go to the integer pipes (symgbMixed), 0 for a
+// kernel that stays on the FP64 pipe alone.  Results are the same bits.
+//   * In levels of 16384 work items up.  Below, a launch leaves most schedulers
+//     without a second warp to share the pipes with and pays for fetching the
+//     longer code: Neo-Hookean 8^3, nine kernels of 10 k items, 41.1 us without
+//     and 43.4 with, of 41 k 69.3 and 53.9; cloth 64 x 64, 7938 items, 41.1 and
+//     40.9; eight small cloth patterns in one graph 206 and 220.
+//   * Templates of 8 FP64 instructions up; lighter ones wait for memory.
+//   * The share that keeps both pipes equally busy: an FP64 instruction of
+//     three register operands holds a scheduler's pipe for 76 cycles (64 with two
+//     of them constants), an integer product its issue slots and pipes for
+//     about 44.
+//   * As many as fit the instruction cache with the rest of the body (32
+//     instructions each, 108 KB in all): cloth 100 x 100 x 64 (plain, 64 x 4),
+//     279 products, 1914 us with none, 1475 with 142 - 158, 1641 with 200, 1677 with
+//     all but powers of two.
+//   * At most 512 in a module, shared out by work: co-resident kernels share
+//     the instruction cache (Neo-Hookean 8^3 x 16, 168 - 261 products in each of
+//     nine templates: 69.3 us with none, 53.4 with 80 each, 63.1 with all), and
+//     NVRTC takes about 7 ms per product.
+std::vector<int> integerProducts(const std::vector<symgb_kernel_desc>& descs, int math, unsigned S) {
+    constexpr std::uint64_t kLeastItems = 1024, kLeastLevelItems = 16384;
+    constexpr int kLeastOps = 8, kCacheInstructions = 6912, kProductInstructions = 32, kModule = 512;
+    constexpr int kFp64Cycles = 76, kProductCycles = 44;
+    struct Count {
+        int muls = 0, fp64 = 0, inner = 0, loads = 0;  // inner: first products of divisions and square roots
+    };
+    std::vector<Count> count(descs.size());
+    std::map<int, std::uint64_t> levelItems;
+    for (std::size_t k = 0; k < descs.size(); ++k) {
+        std::vector<std::uint64_t> loads;
+        Count& c = count[k];
+        for (const LinOp& L : linearCode(descs[k], math, &loads)) {
+            if (L.op == OP_MUL) ++c.muls, ++c.fp64;
+            else if (L.op == OP_FDIV) ++c.inner, c.fp64 += 5;
+            else if (L.op == OP_FSQRT) ++c.inner, c.fp64 += 6;
+            else if (L.op == OP_DIV || L.op == OP_SQRT || L.op == OP_REC) c.fp64 += 9;
+            else if (L.op == OP_FREC) c.fp64 += 4;
+            else if (L.op != OP_LDK && L.op != OP_ST && L.op != OP_MOV && L.op != OP_NEG) ++c.fp64;
+        }
+        c.loads = (int)loads.size();
+        if (c.fp64 >= kLeastOps) levelItems[descs[k].level] += descs[k].num_instances * S;
+    }
+    std::vector<int> take(descs.size(), 0);
+    std::vector<double> work(descs.size(), 0.0);
+    double all = 0.0;
+    int total = 0;
+    for (std::size_t k = 0; k < descs.size(); ++k) {
+        const Count& c = count[k];
+        const std::uint64_t items = descs[k].num_instances * S;
+        if (c.fp64 < kLeastOps || c.muls + c.inner == 0) continue;
+        if (items < kLeastItems || levelItems[descs[k].level] < kLeastLevelItems) continue;
+        const int share = (int)((long long)c.fp64 * kFp64Cycles / (kFp64Cycles + kProductCycles)) - c.inner;
+        const int room = (kCacheInstructions - 3 * (c.fp64 - c.muls) - 6 * c.loads) / kProductInstructions - c.inner;
+        take[k] = std::max(0, std::min({c.muls, share, room}));
+        if (!take[k] && c.inner) take[k] = 1;  // a mixed body for its divisions and square roots
+        total += take[k];
+        work[k] = (double)items * c.fp64;
+        all += work[k];
+    }
+    if (total > kModule)
+        for (std::size_t k = 0; k < descs.size(); ++k)
+            if (take[k]) take[k] = std::min(take[k], std::max(1, (int)(kModule * work[k] / all)));
+    return take;
 }
 
 // Templates of at most this many operations per thread (operations x items)
@@ -235,7 +388,11 @@ constexpr std::size_t kSplitOps = 1024;
 // loads are in flight together.  `split`: threads whose items are all in
 // range take an unguarded copy of the loop (kSplitOps).
 void emitItems(std::ostringstream& os, int k, std::uint64_t total, unsigned S, int tpb, int items, int l2,
-               const std::string& b0, const char* indent, bool split, int order) {
+               const std::string& b0, const char* indent, bool split, int order, bool mixed) {
+    const std::string body = mixed ? "if (symgbMixed" : "symgbBody";
+    const std::string tail = mixed ? ")) symgbRedo" + std::to_string(k) + "<" + std::to_string(l2) + ">(x, xw, p, c, res, dp, w / " +
+                                         std::to_string(S) + "ull, (unsigned)(w % " + std::to_string(S) + "ull))"
+                                   : ")";
     const std::string targs = "<" + std::to_string(l2) + (order ? ", " + std::to_string(order) : std::string()) + ">";
     os << indent << "const unsigned long long w0 = (" << b0 << ") * " << (std::uint64_t)tpb * items
        << "ull + threadIdx.x;\n";
@@ -243,15 +400,18 @@ void emitItems(std::ostringstream& os, int k, std::uint64_t total, unsigned S, i
         os << indent << "if (w0 + " << u64((std::uint64_t)(items - 1) * tpb) << " < " << u64(total) << ") {\n"
            << indent << "    #pragma unroll\n" << indent << "    for (int j = 0; j < " << items << "; ++j) {\n"
            << indent << "        const unsigned long long w = w0 + (unsigned long long)j * " << tpb << "ull;\n"
-           << indent << "        symgbBody" << k << targs << "(x, xw, p, c, res, dp, w / " << S
-           << "ull, (unsigned)(w % " << S << "ull));\n"
+           << indent << "        " << body << k << targs << "(x, xw, p, c, res, dp, w / " << S
+           << "ull, (unsigned)(w % " << S << "ull)" << tail << ";\n"
            << indent << "    }\n" << indent << "} else {\n";
     }
-    if (items > 1) os << indent << "#pragma unroll\n" << indent << "for (int j = 0; j < " << items << "; ++j) {\n";
+    // A heavy mixed body is not unrolled: one copy of it nearly fills the
+    // instruction cache.
+    if (items > 1)
+        os << indent << (mixed && !split ? "#pragma unroll 1\n" : "#pragma unroll\n") << indent << "for (int j = 0; j < " << items << "; ++j) {\n";
     else os << indent << "{\n" << indent << "    const int j = 0;\n";
     os << indent << "    const unsigned long long w = w0 + (unsigned long long)j * " << tpb << "ull;\n"
-       << indent << "    if (w < " << u64(total) << ") symgbBody" << k << targs << "(x, xw, p, c, res, dp, w / "
-       << S << "ull, (unsigned)(w % " << S << "ull));\n"
+       << indent << "    if (w < " << u64(total) << ") {\n" << indent << "        " << body << k << targs << "(x, xw, p, c, res, dp, w / "
+       << S << "ull, (unsigned)(w % " << S << "ull)" << tail << ";\n" << indent << "    }\n"
        << indent << "}\n";
     if (items > 1 && split) os << indent << "}\n";
 }
@@ -292,24 +452,25 @@ void emitGroups(std::ostringstream& os, int k, const symgb_kernel_desc& d, unsig
 
 // The work of kernel k in either item layout.
 void emitWork(std::ostringstream& os, int k, const symgb_kernel_desc& d, std::size_t ops, unsigned S, int tpb,
-              int items, int l2, const std::string& b0, const char* indent, bool grouped, int order = 0) {
+              int items, int l2, const std::string& b0, const char* indent, bool grouped, int order, bool mixed) {
     const bool split = ops * (std::size_t)items <= kSplitOps;
     if (grouped) emitGroups(os, k, d, S, tpb, items, l2, b0, indent, split);
-    else emitItems(os, k, d.num_instances * S, S, tpb, items, l2, b0, indent, split, order);
+    else emitItems(os, k, d.num_instances * S, S, tpb, items, l2, b0, indent, split, order, mixed);
 }
 
 // Dispatch of block `b` over the kernels of one launch (kernel-major block
 // ranges, each kernel's work items in consecutive blocks).
 void emitDispatch(std::ostringstream& os, const std::vector<int>& ks, const std::vector<symgb_kernel_desc>& descs,
                   const std::vector<std::size_t>& opCount, unsigned S, int tpb, int items, int l2, const char* indent,
-                  bool grouped, int order = 0) {
+                  bool grouped, const std::vector<int>& intMuls, int order = 0) {
     std::uint64_t first = 0;
     const std::string inner = std::string(indent) + "    ";
     for (std::size_t q = 0; q < ks.size(); ++q) {
         const int k = ks[q];
         const std::uint64_t blocks = kernelBlocks(descs[k], S, tpb, items, grouped);
         os << indent << (q ? "else " : "") << "if (b < " << u64(first + blocks) << ") {\n";
-        emitWork(os, k, descs[k], opCount[k], S, tpb, items, l2, "b - " + u64(first), inner.c_str(), grouped, order);
+        emitWork(os, k, descs[k], opCount[k], S, tpb, items, l2, "b - " + u64(first), inner.c_str(), grouped, order,
+                 intMuls[k] > 0);
         os << indent << "}\n";
         first += blocks;
     }
@@ -432,13 +593,34 @@ JitSource generateModule(const std::vector<symgb_kernel_desc>& descs, int numLev
               "        v[0] = SYMGB_LD(a);\n"
               "    }\n}\n\n";
     std::vector<std::size_t> opCount(descs.size());
+    // Heavy bodies of a kernel that dispatches over several are functions of
+    // their own: in one, their compile time grows with its square (Neo-Hookean
+    // levels, nine templates of 600 operations: 4.9 -> 1.3 s).
+    constexpr std::size_t kHeavyOps = 200;
+    std::vector<std::size_t> templateOps;
+    int heavy = 0;
+    for (const auto& d : descs) {
+        templateOps.push_back(linearCode(d, cfg.math, nullptr).size());
+        heavy += d.num_instances && templateOps.back() > kHeavyOps;
+    }
+    const bool dispatch = cfg.kind != JIT_PLAIN && !grouped && heavy > 1;
+    const std::vector<int> intMuls = grouped ? std::vector<int>(descs.size(), 0) : integerProducts(descs, cfg.math, S);
     if (!cfg.directBase.empty() && (cfg.directBase.size() != descs.size() || S != 1))
         throw std::runtime_error("codegen: direct result rows need one value set and a row table per kernel");
     for (std::size_t k = 0; k < descs.size(); ++k) {
         const std::vector<std::int64_t>* direct = cfg.directBase.empty() ? nullptr : &cfg.directBase[k];
         if (direct)
             for (std::int64_t b : *direct) out.direct |= b >= 0;
-        opCount[k] = emitBody(os, (int)k, descs[k], cfg.math, S, grouped ? &gt : nullptr, direct);
+        const bool called = dispatch && templateOps[k] > kHeavyOps;
+        opCount[k] = emitBody(os, (int)k, descs[k], cfg.math, S, grouped ? &gt : nullptr, direct, called);
+        if (intMuls[k]) {
+            os << "#ifdef SYMGB_ORDERED\n";
+            emitBody(os, (int)k, descs[k], cfg.math, S, nullptr, direct, called, intMuls[k]);
+            os << "template <int L2>\n__device__ __noinline__ void symgbRedo" << k
+               << "(const double* x, double* xw, const unsigned* p, const double* c, double* res, const unsigned* dp, "
+                  "unsigned long long i, unsigned s) {\n    symgbBody"
+               << k << "<L2>(x, xw, p, c, res, dp, i, s);\n}\n#endif\n\n";
+        }
     }
     const char* params = "(const double* SYMGB_XR x, double* SYMGB_XR xw, const unsigned* __restrict__ p, "
                          "const double* __restrict__ c, double* __restrict__ res, const unsigned* __restrict__ dp";
@@ -463,7 +645,7 @@ JitSource generateModule(const std::vector<symgb_kernel_desc>& descs, int numLev
             os << "extern \"C\" __global__ void " << launchBounds(tpb, cfg.minBlocks) << " " << name << params << ") {\n";
             const int order = emitPrologue(os, o, items == 1 && !grouped);
             emitWork(os, k, descs[k], opCount[k], S, tpb, items, 0, "(unsigned long long)blockIdx.x", "    ", grouped,
-                     order);
+                     order, intMuls[k] > 0);
             emitEpilogue(os, o);
             os << "}\n\n";
             out.launches.push_back({name, k, -1, kernelBlocks(descs[k], S, tpb, items, grouped), tpb, items, false});
@@ -482,7 +664,7 @@ JitSource generateModule(const std::vector<symgb_kernel_desc>& descs, int numLev
             os << "extern \"C\" __global__ void " << launchBounds(tpb, cfg.minBlocks) << " " << name << params << ") {\n";
             const int order = emitPrologue(os, o, items == 1 && !grouped);
             os << "    const unsigned long long b = blockIdx.x;\n";
-            emitDispatch(os, ks, descs, opCount, S, tpb, items, 0, "    ", grouped, order);
+            emitDispatch(os, ks, descs, opCount, S, tpb, items, 0, "    ", grouped, intMuls, order);
             emitEpilogue(os, o);
             os << "}\n\n";
             out.launches.push_back({name, -1, L, blocksOf(ks, descs, S, tpb, items, grouped), tpb, items, false});
@@ -504,7 +686,7 @@ JitSource generateModule(const std::vector<symgb_kernel_desc>& descs, int numLev
             const std::uint64_t nb = blocksOf(ks, descs, S, tpb, items, grouped);
             most = std::max(most, nb);
             os << "    for (unsigned long long b = blockIdx.x; b < " << u64(nb) << "; b += gridDim.x) {\n";
-            emitDispatch(os, ks, descs, opCount, S, tpb, items, firstLevel ? 0 : 1, "        ", grouped);
+            emitDispatch(os, ks, descs, opCount, S, tpb, items, firstLevel ? 0 : 1, "        ", grouped, intMuls);
             os << "    }\n";
             firstLevel = false;
         }

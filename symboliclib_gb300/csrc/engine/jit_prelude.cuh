@@ -8,6 +8,9 @@
 #define SYMGB_ERR_TIMEOUT (-4)
 #endif
 
+// Generated bodies that are functions of their own.
+#define SYMGB_CALLED __noinline__
+
 // Negation flips the sign (C's unary minus; exact, -(+0) = -0).  Written as
 // the language's negation so the compiler can fold it into the sign modifier
 // of the FMA, add or multiply that consumes it: no instruction of its own and
@@ -77,6 +80,71 @@ __device__ __forceinline__ double symgbFastSqrt(double x) {
     g = __fma_rn(__fma_rn(-g, g, x), h, g);
     if (__builtin_expect(symgbSignExp(x) - 123u > 1800u, 0)) g = symgbIeeeSqrt(x);
     return g;
+}
+
+// Double multiplication on the integer pipes, bit-identical to __dmul_rn for
+// operands that are zero or lie in [2^-255, 2^256), and for products of up to
+// four such factors taken in any order (which stay in [2^-1020, 2^1024)).
+// symgbSig is the upper part of a significand (leading bit and 20 bits; 0 for
+// a zero), symgbOutside tells operands the product does not cover.
+// The 53-bit significands are multiplied as 21 + 32 bit halves; the 106-bit
+// product is shifted so that its leading 53 bits fill hi:lo and the next 32 r;
+// rounding to nearest even adds the carry out of r + 0x7fffffff + (lo odd or
+// bits below r).  Sign and exponent fields add as integers, less the bias.
+__device__ __forceinline__ unsigned symgbSig(double a) {
+    const unsigned h = (unsigned)__double2hiint(a);
+    return min(h & 0x7fffffffu, (h & 0xfffffu) | 0x100000u);
+}
+__device__ __forceinline__ bool symgbOutside(double a) {
+    const unsigned t = (unsigned)__double2hiint(a) & 0x7fffffffu;
+    return t - 0x30000000u >= 0x1ff00000u && (t | (unsigned)__double2loint(a)) != 0u;
+}
+__device__ __forceinline__ double symgbMulInt(double a, double b, unsigned am, unsigned bm) {
+    const unsigned ah = (unsigned)__double2hiint(a), al = (unsigned)__double2loint(a);
+    const unsigned bh = (unsigned)__double2hiint(b), bl = (unsigned)__double2loint(b);
+    const unsigned long long t0 = (unsigned long long)al * bl;
+    const unsigned long long t1 = (unsigned long long)am * bl + (t0 >> 32);
+    const unsigned long long t2 = (unsigned long long)al * bm + t1;
+    const unsigned long long t3 = (unsigned long long)am * bm + (t2 >> 32);
+    const unsigned p0 = (unsigned)t0, p1 = (unsigned)t2, p2 = (unsigned)t3, p3 = (unsigned)(t3 >> 32);
+    const unsigned k = p3 >> 9, n = 12u - k;  // product of significands in [2, 4) or [1, 2)
+    const unsigned hi = __funnelshift_l(p2, p3, n), lo = __funnelshift_l(p1, p2, n), r = __funnelshift_l(p0, p1, n);
+    const unsigned long long up = ((unsigned long long)r + 0x7fffffffu + (((lo & 1u) | p0) ? 1u : 0u)) >> 32;
+    const unsigned e = (ah - am) + (bh - bm) + k * 0x100000u + 0xc0200000u;  // sign and exponent, less hi's leading bit
+    const unsigned long long m = (((unsigned long long)hi << 32) | lo) + up + ((unsigned long long)e << 32);
+    unsigned rh = (unsigned)(m >> 32);
+    if (p3 == 0u) rh = (ah ^ bh) & 0x80000000u;  // a zero factor (the low word is zero then)
+    return __hiloint2double((int)rh, (int)(unsigned)m);
+}
+// symgbFastDiv with its first product on the integer pipes (a as for
+// symgbMulInt); `outside` where that does not cover the reciprocal.
+__device__ __forceinline__ double symgbFastDivInt(double a, double b, unsigned am, bool& outside) {
+    const double r0 = symgbRcpApprox(b);
+    const double r = __fma_rn(r0, __fma_rn(-b, r0, 1.0), r0);
+    outside |= symgbOutside(r);
+    const double q0 = symgbMulInt(a, r, am, symgbSig(r));
+    double q = __fma_rn(r, __fma_rn(-b, q0, a), q0);
+    const bool zeroA = am == 0u;
+    if (zeroA) q = q0;
+    outside |= (symgbSignExp(b) & 0x7ffu) - 523u > 1000u;
+    return q;
+}
+// a * (-1)^NEG 2^K for the same operands (|K| <= 64): the exponent field moves by K.
+template <int K, int NEG>
+__device__ __forceinline__ double symgbMulPow2(double a) {
+    const unsigned h = (unsigned)__double2hiint(a);
+    const unsigned q = (h & 0x7fffffffu) ? h + ((unsigned)K << 20) : h;
+    return __hiloint2double((int)(NEG ? q ^ 0x80000000u : q), __double2loint(a));
+}
+
+// symgbFastSqrt with its two products on the integer pipes (x as for symgbMulInt).
+__device__ __forceinline__ double symgbFastSqrtInt(double x, unsigned xm, bool& outside) {
+    const double y = symgbRsqrtApprox(x);
+    outside |= symgbOutside(y);  // of a zero, negative or NaN x too
+    double g = symgbMulInt(x, y, xm, symgbSig(y));
+    const double h = symgbMulPow2<-1, 0>(y);
+    g = __fma_rn(g, __fma_rn(-g, h, 0.5), g);
+    return __fma_rn(__fma_rn(-g, g, x), h, g);
 }
 
 __device__ __forceinline__ unsigned long long symgbGlobalTimerNs() {
