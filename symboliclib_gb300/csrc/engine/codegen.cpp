@@ -21,6 +21,7 @@
 #include "codegen.hpp"
 
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <map>
 #include <set>
@@ -57,6 +58,20 @@ const char* libName(int op) {
     }
 }
 
+// Some of a template's output rows with the operations and loads they need
+// (splitTemplate); a thread evaluates one piece of one work item.
+struct Piece {
+    std::vector<char> ops, loads;  // by linear operation, by load
+    double cost = 0.0;             // FP64 instructions
+};
+
+// The device function of a piece, as the dispatch calls it.
+struct Call {
+    std::string body;  // symgbBody<k>, symgbMixed<k> or symgbPart<k>_<piece>
+    std::size_t ops = 0;  // operations of the whole template
+    bool mixed = false;
+};
+
 // Emits the device function evaluating kernel k.
 //   Strided items (grouped == nullptr): symgbBody<k><L2, ORDER>(..., i, s)
 //     evaluates one work item (instance i, value set s) and loads its own index
@@ -80,19 +95,30 @@ const char* libName(int op) {
 //     results again.  A product's range is checked at its factors that come
 //     from loads or FP64 instructions, once each; products of up to four of
 //     them need no check.
+//   With `piece`: symgbPart<k>_<pieceIndex>, the strided body of those rows.
 // `called`: emitted as a function of its own instead of into its callers.
 std::size_t emitBody(std::ostringstream& os, int k, const symgb_kernel_desc& d, int math, unsigned S,
                      const GroupedTables* grouped, const std::vector<std::int64_t>* direct, bool called,
-                     int intMuls = 0) {
+                     int intMuls = 0, const Piece* piece = nullptr, int pieceIndex = 0) {
     std::vector<std::uint64_t> loads;
-    const std::vector<LinOp> ops = linearCode(d, math, &loads);
+    std::vector<LinOp> ops = linearCode(d, math, &loads);
+    if (piece) {
+        std::vector<std::uint64_t> l;
+        std::vector<LinOp> o;
+        for (std::size_t j = 0; j < loads.size(); ++j)
+            if (piece->loads[j]) l.push_back(loads[j]);
+        for (std::size_t j = 0; j < ops.size(); ++j)
+            if (piece->ops[j]) o.push_back(ops[j]);
+        loads.swap(l);
+        ops.swap(o);
+    }
     const std::uint64_t n = d.num_instances;
     const bool g = grouped != nullptr;
     const char* in = g ? "        " : "    ";
     const bool mixed = intMuls > 0;
-    if (!mixed) os << "// kernel " << k << ": " << n << " instances, level " << d.level << ", " << loads.size() << " loads, "
+    if (!mixed && !piece) os << "// kernel " << k << ": " << n << " instances, level " << d.level << ", " << loads.size() << " loads, "
        << ops.size() << " operations\n";
-    if (called && !mixed) os << "#ifndef SYMGB_CALLED\n#define SYMGB_CALLED\n#endif\n";
+    if (called && !mixed && !piece) os << "#ifndef SYMGB_CALLED\n#define SYMGB_CALLED\n#endif\n";
     if (g)
         os << "template <int L2, int IT, bool FULL>\n__device__ __forceinline__ void symgbGroup" << k
            << "(const double* SYMGB_XR x, double* SYMGB_XR xw, const unsigned* __restrict__ p, "
@@ -100,7 +126,8 @@ std::size_t emitBody(std::ostringstream& os, int k, const symgb_kernel_desc& d, 
               "unsigned long long g, unsigned s) {\n";
     else
         os << "template <int L2, int ORDER = 0>\n__device__ " << (called ? "SYMGB_CALLED " : "__forceinline__ ")
-           << (mixed ? "bool symgbMixed" : "void symgbBody") << k
+           << (mixed ? "bool symgbMixed" : piece ? "void symgbPart" : "void symgbBody") << k
+           << (piece ? "_" + std::to_string(pieceIndex) : std::string())
            << "(const double* SYMGB_XR x, double* SYMGB_XR xw, const unsigned* __restrict__ p, "
               "const double* __restrict__ c, double* __restrict__ res, const unsigned* __restrict__ dp, "
               "unsigned long long i, unsigned s) {\n";
@@ -307,6 +334,23 @@ std::size_t emitBody(std::ostringstream& os, int k, const symgb_kernel_desc& d, 
     return ops.size();
 }
 
+std::uint64_t blocksFor(std::uint64_t total, int tpb, int items) {
+    const std::uint64_t per = (std::uint64_t)tpb * items;
+    return (total + per - 1) / per;
+}
+
+// FP64 instructions of an operation.
+int fp64Cost(int op) {
+    switch (op) {
+        case OP_LDK: case OP_ST: case OP_MOV: case OP_NEG: return 0;
+        case OP_FDIV: return 5;
+        case OP_FSQRT: return 6;
+        case OP_FREC: return 4;
+        case OP_DIV: case OP_SQRT: case OP_REC: return 9;
+        default: return 1;
+    }
+}
+
 // Products of every kernel that go to the integer pipes (symgbMixed), 0 for a
 // kernel that stays on the FP64 pipe alone.  Results are the same bits.
 //   * In levels of 16384 work items up.  Below, a launch leaves most schedulers
@@ -340,12 +384,9 @@ std::vector<int> integerProducts(const std::vector<symgb_kernel_desc>& descs, in
         std::vector<std::uint64_t> loads;
         Count& c = count[k];
         for (const LinOp& L : linearCode(descs[k], math, &loads)) {
-            if (L.op == OP_MUL) ++c.muls, ++c.fp64;
-            else if (L.op == OP_FDIV) ++c.inner, c.fp64 += 5;
-            else if (L.op == OP_FSQRT) ++c.inner, c.fp64 += 6;
-            else if (L.op == OP_DIV || L.op == OP_SQRT || L.op == OP_REC) c.fp64 += 9;
-            else if (L.op == OP_FREC) c.fp64 += 4;
-            else if (L.op != OP_LDK && L.op != OP_ST && L.op != OP_MOV && L.op != OP_NEG) ++c.fp64;
+            c.muls += L.op == OP_MUL;
+            c.inner += L.op == OP_FDIV || L.op == OP_FSQRT;
+            c.fp64 += fp64Cost(L.op);
         }
         c.loads = (int)loads.size();
         if (c.fp64 >= kLeastOps) levelItems[descs[k].level] += descs[k].num_instances * S;
@@ -373,6 +414,157 @@ std::vector<int> integerProducts(const std::vector<symgb_kernel_desc>& descs, in
     return take;
 }
 
+// A template's output rows with everything each of them needs.
+struct Rows {
+    int ops = 0, loads = 0;
+    struct Row {
+        std::vector<int> ops, loads;  // operations (its store among them) and loads it needs
+        int cost = 0;
+    };
+    std::vector<Row> rows;   // in template order; empty where a row is stored twice
+    std::vector<int> cost;   // by operation
+};
+
+Rows rowsOf(const symgb_kernel_desc& d, int math) {
+    std::vector<std::uint64_t> loads;
+    const std::vector<LinOp> ops = linearCode(d, math, &loads);
+    Rows r;
+    r.ops = (int)ops.size();
+    r.loads = (int)loads.size();
+    std::vector<int> def(256, -1);  // register -> load (0 .. loads - 1) or operation (loads + j) that wrote it
+    for (int i = 0; i < r.loads; ++i) def[(loads[i] >> 8) & 0xff] = i;
+    std::vector<std::vector<int>> needs(r.ops);
+    std::vector<char> stored(d.num_output_rows, 0);
+    for (int j = 0; j < r.ops; ++j) {
+        for (int q = 0; q < ops[j].nsrc; ++q) needs[j].push_back(def[ops[j].src[q]]);
+        if (ops[j].d >= 0) def[ops[j].d] = r.loads + j;
+        r.cost.push_back(fp64Cost(ops[j].op));
+    }
+    std::vector<int> seen(r.ops + r.loads, -1);
+    for (int j = 0; j < r.ops; ++j) {
+        if (ops[j].op != OP_ST) continue;
+        if (ops[j].row >= stored.size() || stored[ops[j].row]) return Rows();
+        stored[ops[j].row] = 1;
+        Rows::Row row;
+        std::vector<int> todo{r.loads + j};
+        while (!todo.empty()) {
+            const int v = todo.back();
+            todo.pop_back();
+            if (v < 0 || seen[v] == j) continue;
+            seen[v] = j;
+            if (v < r.loads) {
+                row.loads.push_back(v);
+                continue;
+            }
+            row.ops.push_back(v - r.loads);
+            row.cost += r.cost[v - r.loads];
+            todo.insert(todo.end(), needs[v - r.loads].begin(), needs[v - r.loads].end());
+        }
+        r.rows.push_back(std::move(row));
+    }
+    return r;
+}
+
+// Cuts a template into `count` pieces: the cheapest piece so far takes the row
+// that adds least to it (of equals the dearest), until all are taken.
+std::vector<Piece> splitTemplate(const Rows& r, int count) {
+    std::vector<Piece> ps(count, Piece{std::vector<char>(r.ops, 0), std::vector<char>(r.loads, 0), 0.0});
+    std::vector<char> taken(r.rows.size(), 0);
+    for (std::size_t left = r.rows.size(); left > 0; --left) {
+        Piece* p = &ps[0];
+        for (Piece& q : ps)
+            if (q.cost < p->cost) p = &q;
+        int row = -1, least = 0;
+        for (std::size_t i = 0; i < r.rows.size(); ++i) {
+            if (taken[i]) continue;
+            int more = 0;
+            for (int j : r.rows[i].ops)
+                if (!p->ops[j]) more += r.cost[j];
+            if (row < 0 || more < least || (more == least && r.rows[i].cost > r.rows[row].cost)) {
+                row = (int)i;
+                least = more;
+            }
+        }
+        taken[row] = 1;
+        p->cost += least;
+        for (int j : r.rows[row].ops) p->ops[j] = 1;
+        for (int j : r.rows[row].loads) p->loads[j] = 1;
+    }
+    return ps;
+}
+
+// Pieces of every kernel's template (empty: whole).  Heavy templates of
+// launches that leave schedulers idle are cut, the pieces going to different
+// blocks: an FP64 instruction takes a warp's scheduler 64 cycles whatever else
+// the warp has ready, so a launch of few warps lasts as long as its longest
+// template, and a shorter one helps although the pieces evaluate shared
+// operations again.  Per level the number of pieces with the shortest estimate,
+// where it is at least a tenth below that of fewer: the longest piece times the
+// blocks that come to lie on one SM.  Blocks are dealt out evenly to GPCs of
+// uneven size, so that from 117 blocks of four warps on (cloth 60 and 62, two
+// pieces exact: 117 blocks and 118, 30.7 and 53.4 us), in a persistent grid of
+// two blocks per SM from 59 on, some SM has two.  GB300, levels: cloth 64 x 64
+// 33.8 -> 27.9 us (three pieces), cloth 20 x 20 31.3 -> 15.6 (six), Neo-Hookean
+// 8^3 x 4 33.1 -> 27.6 (two), 4^3 exact 37.1 -> 12.8 (eight).
+std::vector<std::vector<Piece>> templatePieces(const std::vector<symgb_kernel_desc>& descs, const JitConfig& cfg,
+                                               const std::vector<int>& intMuls) {
+    constexpr int kHeavy = 64;  // FP64 instructions
+    constexpr double kRounds = 4.0, kAlone = 1.15;  // a warp alone on its scheduler also waits for its loads
+    const double oneRound = cfg.kind == JIT_PERSISTENT ? 58.0 : 116.0;  // blocks of four warps
+    std::vector<std::vector<Piece>> out(descs.size());
+    std::map<int, std::vector<int>> heavy;  // by level
+    std::vector<int> costs(descs.size(), 0);
+    for (std::size_t k = 0; k < descs.size(); ++k) {
+        if (!descs[k].num_instances || intMuls[k]) continue;
+        for (const LinOp& L : linearCode(descs[k], cfg.math, nullptr)) costs[k] += fp64Cost(L.op);
+        if (costs[k] >= kHeavy) heavy[descs[k].level].push_back((int)k);
+    }
+    for (const auto& level : heavy) {
+        // Blocks of four warps of kernel k's work items, per piece.
+        auto blocks = [&](int k) {
+            const int tpb = cfg.kind == JIT_PLAIN ? cfg.kernelTpb.at(k)
+                                                  : cfg.levelTpb.at(cfg.kind == JIT_LEVELS ? level.first : 0);
+            const int items = cfg.kind == JIT_PLAIN ? cfg.kernelItems.at(k)
+                                                    : cfg.levelItems.at(cfg.kind == JIT_LEVELS ? level.first : 0);
+            return (double)blocksFor(descs[k].num_instances * cfg.numSets, tpb, items) * tpb / 128.0;
+        };
+        auto estimate = [&](const std::vector<std::vector<Piece>>& ps) {
+            double longest = 0.0, all = 0.0, count = 0.0;
+            for (std::size_t i = 0; i < ps.size(); ++i) {
+                const int k = level.second[i];
+                double most = ps[i].empty() ? (double)costs[k] : 0.0, sum = most;
+                for (const Piece& q : ps[i]) {
+                    most = std::max(most, q.cost);
+                    sum += q.cost;
+                }
+                longest = std::max(longest, most);
+                all += sum * blocks(k);
+                count += std::max<std::size_t>(1, ps[i].size()) * blocks(k);
+            }
+            const double rounds = std::ceil(count / oneRound);
+            return rounds <= 1.0 ? kAlone * longest : longest + std::min(rounds - 1.0, count / oneRound) * all / count;
+        };
+        std::vector<std::vector<Piece>> best(level.second.size());
+        double bound = estimate(best);
+        double count = 0.0;
+        for (int k : level.second) count += blocks(k);
+        if (count > kRounds * oneRound) continue;  // the chip is full
+        std::vector<Rows> rows;
+        for (int k : level.second) rows.push_back(rowsOf(descs[k], cfg.math));
+        for (int pieces : {2, 3, 4, 6, 8}) {
+            std::vector<std::vector<Piece>> ps(rows.size());
+            for (std::size_t i = 0; i < rows.size(); ++i)
+                if (rows[i].rows.size() >= (std::size_t)pieces) ps[i] = splitTemplate(rows[i], pieces);
+            const double t = estimate(ps);
+            if (t > 0.9 * bound) continue;
+            bound = t;
+            best.swap(ps);
+        }
+        for (std::size_t i = 0; i < best.size(); ++i) out[level.second[i]].swap(best[i]);
+    }
+    return out;
+}
+
 // Templates of at most this many operations per thread (operations x items)
 // get a second, unguarded copy of the items loop for threads whose items are
 // all in range: without a bounds check per item the compiler can issue every
@@ -387,9 +579,10 @@ constexpr std::size_t kSplitOps = 1024;
 // each of the thread's rounds (coalesced), rounds unrolled so the items'
 // loads are in flight together.  `split`: threads whose items are all in
 // range take an unguarded copy of the loop (kSplitOps).
-void emitItems(std::ostringstream& os, int k, std::uint64_t total, unsigned S, int tpb, int items, int l2,
-               const std::string& b0, const char* indent, bool split, int order, bool mixed) {
-    const std::string body = mixed ? "if (symgbMixed" : "symgbBody";
+void emitItems(std::ostringstream& os, int k, const Call& call, std::uint64_t total, unsigned S, int tpb, int items,
+               int l2, const std::string& b0, const char* indent, bool split, int order) {
+    const bool mixed = call.mixed;
+    const std::string body = (mixed ? "if (" : "") + call.body;
     const std::string tail = mixed ? ")) symgbRedo" + std::to_string(k) + "<" + std::to_string(l2) + ">(x, xw, p, c, res, dp, w / " +
                                          std::to_string(S) + "ull, (unsigned)(w % " + std::to_string(S) + "ull))"
                                    : ")";
@@ -400,7 +593,7 @@ void emitItems(std::ostringstream& os, int k, std::uint64_t total, unsigned S, i
         os << indent << "if (w0 + " << u64((std::uint64_t)(items - 1) * tpb) << " < " << u64(total) << ") {\n"
            << indent << "    #pragma unroll\n" << indent << "    for (int j = 0; j < " << items << "; ++j) {\n"
            << indent << "        const unsigned long long w = w0 + (unsigned long long)j * " << tpb << "ull;\n"
-           << indent << "        " << body << k << targs << "(x, xw, p, c, res, dp, w / " << S
+           << indent << "        " << body << targs << "(x, xw, p, c, res, dp, w / " << S
            << "ull, (unsigned)(w % " << S << "ull)" << tail << ";\n"
            << indent << "    }\n" << indent << "} else {\n";
     }
@@ -410,15 +603,10 @@ void emitItems(std::ostringstream& os, int k, std::uint64_t total, unsigned S, i
         os << indent << (mixed && !split ? "#pragma unroll 1\n" : "#pragma unroll\n") << indent << "for (int j = 0; j < " << items << "; ++j) {\n";
     else os << indent << "{\n" << indent << "    const int j = 0;\n";
     os << indent << "    const unsigned long long w = w0 + (unsigned long long)j * " << tpb << "ull;\n"
-       << indent << "    if (w < " << u64(total) << ") {\n" << indent << "        " << body << k << targs << "(x, xw, p, c, res, dp, w / "
+       << indent << "    if (w < " << u64(total) << ") {\n" << indent << "        " << body << targs << "(x, xw, p, c, res, dp, w / "
        << S << "ull, (unsigned)(w % " << S << "ull)" << tail << ";\n" << indent << "    }\n"
        << indent << "}\n";
     if (items > 1 && split) os << indent << "}\n";
-}
-
-std::uint64_t blocksFor(std::uint64_t total, int tpb, int items) {
-    const std::uint64_t per = (std::uint64_t)tpb * items;
-    return (total + per - 1) / per;
 }
 
 // Blocks of kernel k: strided, n*S work items at tpb*items per block;
@@ -451,35 +639,35 @@ void emitGroups(std::ostringstream& os, int k, const symgb_kernel_desc& d, unsig
 }
 
 // The work of kernel k in either item layout.
-void emitWork(std::ostringstream& os, int k, const symgb_kernel_desc& d, std::size_t ops, unsigned S, int tpb,
-              int items, int l2, const std::string& b0, const char* indent, bool grouped, int order, bool mixed) {
-    const bool split = ops * (std::size_t)items <= kSplitOps;
+void emitWork(std::ostringstream& os, int k, const symgb_kernel_desc& d, const Call& call, unsigned S, int tpb,
+              int items, int l2, const std::string& b0, const char* indent, bool grouped, int order) {
+    const bool split = call.ops * (std::size_t)items <= kSplitOps;
     if (grouped) emitGroups(os, k, d, S, tpb, items, l2, b0, indent, split);
-    else emitItems(os, k, d.num_instances * S, S, tpb, items, l2, b0, indent, split, order, mixed);
+    else emitItems(os, k, call, d.num_instances * S, S, tpb, items, l2, b0, indent, split, order);
 }
 
 // Dispatch of block `b` over the kernels of one launch (kernel-major block
-// ranges, each kernel's work items in consecutive blocks).
+// ranges, each piece's work items in consecutive blocks).
 void emitDispatch(std::ostringstream& os, const std::vector<int>& ks, const std::vector<symgb_kernel_desc>& descs,
-                  const std::vector<std::size_t>& opCount, unsigned S, int tpb, int items, int l2, const char* indent,
-                  bool grouped, const std::vector<int>& intMuls, int order = 0) {
+                  const std::vector<std::vector<Call>>& calls, unsigned S, int tpb, int items, int l2,
+                  const char* indent, bool grouped, int order = 0) {
     std::uint64_t first = 0;
     const std::string inner = std::string(indent) + "    ";
-    for (std::size_t q = 0; q < ks.size(); ++q) {
-        const int k = ks[q];
+    for (int k : ks) {
         const std::uint64_t blocks = kernelBlocks(descs[k], S, tpb, items, grouped);
-        os << indent << (q ? "else " : "") << "if (b < " << u64(first + blocks) << ") {\n";
-        emitWork(os, k, descs[k], opCount[k], S, tpb, items, l2, "b - " + u64(first), inner.c_str(), grouped, order,
-                 intMuls[k] > 0);
-        os << indent << "}\n";
-        first += blocks;
+        for (const Call& call : calls[k]) {
+            os << indent << (first ? "else " : "") << "if (b < " << u64(first + blocks) << ") {\n";
+            emitWork(os, k, descs[k], call, S, tpb, items, l2, "b - " + u64(first), inner.c_str(), grouped, order);
+            os << indent << "}\n";
+            first += blocks;
+        }
     }
 }
 
-std::uint64_t blocksOf(const std::vector<int>& ks, const std::vector<symgb_kernel_desc>& descs, unsigned S, int tpb,
-                       int items, bool grouped) {
+std::uint64_t blocksOf(const std::vector<int>& ks, const std::vector<symgb_kernel_desc>& descs,
+                       const std::vector<std::vector<Call>>& calls, unsigned S, int tpb, int items, bool grouped) {
     std::uint64_t b = 0;
-    for (int k : ks) b += kernelBlocks(descs[k], S, tpb, items, grouped);
+    for (int k : ks) b += kernelBlocks(descs[k], S, tpb, items, grouped) * calls[k].size();
     return b;
 }
 
@@ -592,27 +780,31 @@ JitSource generateModule(const std::vector<symgb_kernel_desc>& descs, int numLev
               "    } else {\n"
               "        v[0] = SYMGB_LD(a);\n"
               "    }\n}\n\n";
-    std::vector<std::size_t> opCount(descs.size());
     // Heavy bodies of a kernel that dispatches over several are functions of
     // their own: in one, their compile time grows with its square (Neo-Hookean
     // levels, nine templates of 600 operations: 4.9 -> 1.3 s).
     constexpr std::size_t kHeavyOps = 200;
+    const std::vector<int> intMuls = grouped ? std::vector<int>(descs.size(), 0) : integerProducts(descs, cfg.math, S);
+    std::vector<std::vector<Piece>> pieces(descs.size());
+    if (!grouped) pieces = templatePieces(descs, cfg, intMuls);
     std::vector<std::size_t> templateOps;
-    int heavy = 0;
-    for (const auto& d : descs) {
-        templateOps.push_back(linearCode(d, cfg.math, nullptr).size());
-        heavy += d.num_instances && templateOps.back() > kHeavyOps;
+    std::size_t heavy = 0;
+    for (std::size_t k = 0; k < descs.size(); ++k) {
+        templateOps.push_back(linearCode(descs[k], cfg.math, nullptr).size());
+        if (descs[k].num_instances && templateOps[k] > kHeavyOps) heavy += std::max<std::size_t>(1, pieces[k].size());
     }
     const bool dispatch = cfg.kind != JIT_PLAIN && !grouped && heavy > 1;
-    const std::vector<int> intMuls = grouped ? std::vector<int>(descs.size(), 0) : integerProducts(descs, cfg.math, S);
     if (!cfg.directBase.empty() && (cfg.directBase.size() != descs.size() || S != 1))
         throw std::runtime_error("codegen: direct result rows need one value set and a row table per kernel");
+    std::vector<std::vector<Call>> calls(descs.size());
     for (std::size_t k = 0; k < descs.size(); ++k) {
         const std::vector<std::int64_t>* direct = cfg.directBase.empty() ? nullptr : &cfg.directBase[k];
         if (direct)
             for (std::int64_t b : *direct) out.direct |= b >= 0;
         const bool called = dispatch && templateOps[k] > kHeavyOps;
-        opCount[k] = emitBody(os, (int)k, descs[k], cfg.math, S, grouped ? &gt : nullptr, direct, called);
+        const std::string id = std::to_string(k);
+        const std::size_t ops =
+            emitBody(os, (int)k, descs[k], cfg.math, S, grouped ? &gt : nullptr, direct, called);
         if (intMuls[k]) {
             os << "#ifdef SYMGB_ORDERED\n";
             emitBody(os, (int)k, descs[k], cfg.math, S, nullptr, direct, called, intMuls[k]);
@@ -620,6 +812,16 @@ JitSource generateModule(const std::vector<symgb_kernel_desc>& descs, int numLev
                << "(const double* x, double* xw, const unsigned* p, const double* c, double* res, const unsigned* dp, "
                   "unsigned long long i, unsigned s) {\n    symgbBody"
                << k << "<L2>(x, xw, p, c, res, dp, i, s);\n}\n#endif\n\n";
+            calls[k].push_back({"symgbMixed" + id, ops, true});
+        } else if (pieces[k].size() > 1) {
+            os << "#ifdef SYMGB_ORDERED\n";
+            for (std::size_t q = 0; q < pieces[k].size(); ++q) {
+                emitBody(os, (int)k, descs[k], cfg.math, S, nullptr, direct, called, 0, &pieces[k][q], (int)q);
+                calls[k].push_back({"symgbPart" + id + "_" + std::to_string(q), ops, false});
+            }
+            os << "#endif\n\n";
+        } else {
+            calls[k].push_back({"symgbBody" + id, ops, false});
         }
     }
     const char* params = "(const double* SYMGB_XR x, double* SYMGB_XR xw, const unsigned* __restrict__ p, "
@@ -644,11 +846,11 @@ JitSource generateModule(const std::vector<symgb_kernel_desc>& descs, int numLev
                                 q + 1 < ks.size() && descs[ks[q + 1]].level == level};
             os << "extern \"C\" __global__ void " << launchBounds(tpb, cfg.minBlocks) << " " << name << params << ") {\n";
             const int order = emitPrologue(os, o, items == 1 && !grouped);
-            emitWork(os, k, descs[k], opCount[k], S, tpb, items, 0, "(unsigned long long)blockIdx.x", "    ", grouped,
-                     order, intMuls[k] > 0);
+            os << "    const unsigned long long b = blockIdx.x;\n";
+            emitDispatch(os, {k}, descs, calls, S, tpb, items, 0, "    ", grouped, order);
             emitEpilogue(os, o);
             os << "}\n\n";
-            out.launches.push_back({name, k, -1, kernelBlocks(descs[k], S, tpb, items, grouped), tpb, items, false});
+            out.launches.push_back({name, k, -1, blocksOf({k}, descs, calls, S, tpb, items, grouped), tpb, items, false});
         }
     } else if (cfg.kind == JIT_LEVELS) {
         const LaunchOrder o{true, false};
@@ -664,10 +866,10 @@ JitSource generateModule(const std::vector<symgb_kernel_desc>& descs, int numLev
             os << "extern \"C\" __global__ void " << launchBounds(tpb, cfg.minBlocks) << " " << name << params << ") {\n";
             const int order = emitPrologue(os, o, items == 1 && !grouped);
             os << "    const unsigned long long b = blockIdx.x;\n";
-            emitDispatch(os, ks, descs, opCount, S, tpb, items, 0, "    ", grouped, intMuls, order);
+            emitDispatch(os, ks, descs, calls, S, tpb, items, 0, "    ", grouped, order);
             emitEpilogue(os, o);
             os << "}\n\n";
-            out.launches.push_back({name, -1, L, blocksOf(ks, descs, S, tpb, items, grouped), tpb, items, false});
+            out.launches.push_back({name, -1, L, blocksOf(ks, descs, calls, S, tpb, items, grouped), tpb, items, false});
         }
     } else if (cfg.kind == JIT_PERSISTENT) {
         const int tpb = cfg.levelTpb.at(0);
@@ -683,10 +885,10 @@ JitSource generateModule(const std::vector<symgb_kernel_desc>& descs, int numLev
             if (ks.empty()) continue;
             if (!firstLevel)
                 os << "    if (!symgbGridBarrier(bar, hostError, timeoutNs, gridDim.x + extra)) return;\n";
-            const std::uint64_t nb = blocksOf(ks, descs, S, tpb, items, grouped);
+            const std::uint64_t nb = blocksOf(ks, descs, calls, S, tpb, items, grouped);
             most = std::max(most, nb);
             os << "    for (unsigned long long b = blockIdx.x; b < " << u64(nb) << "; b += gridDim.x) {\n";
-            emitDispatch(os, ks, descs, opCount, S, tpb, items, firstLevel ? 0 : 1, "        ", grouped, intMuls);
+            emitDispatch(os, ks, descs, calls, S, tpb, items, firstLevel ? 0 : 1, "        ", grouped);
             os << "    }\n";
             firstLevel = false;
         }
