@@ -59,25 +59,36 @@ DEFAULT = Sched("levels", 1, 128, 1, 1, "compiled")
 
 
 def time_schedule(unit: native.Unit, sched: Sched, stream, flush=None, runs: int = 5, warmup: int = 2) -> float:
-    """Median microseconds of one run under `sched` (CUDA events on the unit's stream)."""
+    """Median microseconds of one run under `sched` (CUDA events on the unit's
+    stream).  Short runs are timed several at a time, launch after launch,
+    where nothing is to be done between them: completions, of graphs too, are
+    seen in steps of 2 us, a tenth of a small unit's run and more than most
+    schedules differ by."""
     import torch
-    sched.apply(unit)
+    sched.apply(unit, graph=0 if flush is None else 1)
     lib = native.symgb()
+
+    def timed(n):
+        if flush is not None:
+            flush.fill_(1.0)
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record(stream)
+        for _ in range(n):
+            native.check(lib.symgb_run_async(unit.handle))
+        b.record(stream)
+        return a, b
     with torch.cuda.stream(stream):
         for _ in range(warmup):
             native.check(lib.symgb_run_async(unit.handle))
-        ts = []
-        for _ in range(runs):
-            if flush is not None:
-                flush.fill_(1.0)
-            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-            a.record(stream)
-            native.check(lib.symgb_run_async(unit.handle))
-            b.record(stream)
-            ts.append((a, b))
+        n = 1
+        if flush is None:
+            a, b = timed(1)
+            torch.cuda.synchronize()
+            n = max(1, min(16, int(0.2 / max(1e-3, a.elapsed_time(b)))))
+        ts = [timed(n) for _ in range(runs)]
         torch.cuda.synchronize()
     native.check(lib.symgb_synchronize(unit.handle))
-    return float(np.median([a.elapsed_time(b) for a, b in ts]) * 1e3)
+    return float(np.median([a.elapsed_time(b) for a, b in ts]) * 1e3) / n
 
 
 def bind_stream(unit: native.Unit):
