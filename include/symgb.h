@@ -108,7 +108,9 @@ typedef struct symgb_schedule {
                                    executor: > 0 is the minimum of resident CTAs per SM its
                                    kernels are compiled for (__launch_bounds__), which caps their
                                    registers; 0 = the compiler's choice */
-    int32_t use_graph;          /* capture run() into a CUDA graph and replay it */
+    int32_t use_graph;          /* capture run() into a CUDA graph at its first run and replay it
+                                   (runs of six or more launches are replayed from their second
+                                   time on in any case) */
     int32_t items_per_thread;   /* work items per thread per pass: 1, 2 or 4 (0 = 1) */
     int32_t fusion_depth;       /* LEVELS: consecutive levels per launch (0/1 = one level; a
                                    group of several levels is one cooperative launch) */
@@ -127,7 +129,10 @@ typedef struct symgb_schedule {
  *     for the process; consecutive launches overlap their start-up
  *     (programmatic dependent launch).  A thread takes items_per_thread work
  *     items (1, 2 or 4, unrolled); lanes_per_item, items_per_tile and
- *     fusion_depth do not apply.
+ *     fusion_depth do not apply.  In launches that fill the chip part of a
+ *     template's products run on the integer pipes, in small ones a heavy
+ *     template's output rows are shared out over several threads; both give
+ *     the same bits.
  *   INTERPRETER: one precompiled kernel runs every template as a bundled
  *     register-machine program (no run-time compilation). */
 #define SYMGB_EXEC_COMPILED 0
