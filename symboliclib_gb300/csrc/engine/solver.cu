@@ -687,6 +687,8 @@ static void place(symgb_solver_t s, const double* values, cudaStream_t st) {
 // sets alone would leave a warp's reads scattered over its 32 rows; more, up
 // to a warp, while the threads fill less than half the chip (rows of 39 entries,
 // BiCGSTAB, 4800 rows x 8 sets: 36 us an iteration with one, 28 with four).
+// Only rows shared by lanes need a power of two of threads: 18.7 k rows x 5
+// sets take 40.9 us a CG iteration with 8 threads to a row, 28.1 with 5.
 static void product(symgb_solver_t s, const double* z, const double* w, double* y, double* d1, double* d2, double* zero,
                     double* zero2, cudaStream_t st) {
     unsigned width = 1;
@@ -696,7 +698,7 @@ static void product(symgb_solver_t s, const double* z, const double* w, double* 
     const std::uint64_t room = (std::uint64_t)s->smCount * 1024;
     const bool wide = width * lanes <= 32 && s->n * width * lanes <= room;
     while (wide && width * lanes < 32 && s->n * width * lanes * 2 <= room) lanes *= 2;
-    if (!wide) width = s->S;
+    if (lanes == 1 || !wide) width = s->S;
     auto launch = [&](auto fn) {
         launchStep(fn, s->blocks(s->n, wide ? 1024 : 2048, width, lanes), s->threads, s->sharedBytes(), st,
                    s->rowPtr.ptr, s->entry.ptr, s->vals.ptr, z, s->n, s->S, width, lanes, w, y, d1, d2, zero, zero2);

@@ -46,6 +46,31 @@ def test_multiply(n, sets, lower):
         assert np.all(np.abs(q[s] - A @ p[s]) <= 2 * n * 2.0 ** -53 * (np.abs(A) @ np.abs(p[s])))
 
 
+@pytest.mark.parametrize("sets,n", [(3, 19456), (3, 19457), (3, 30001), (3, 38913), (5, 9728), (5, 9729), (5, 19456),
+                                    (5, 19457), (7, 12345), (11, 5000), (33, 5003)])
+def test_multiply_many_rows(sets, n):
+    """Row counts around which a row's threads change; at most 9 terms a row, either summation order."""
+    torch = pytest.importorskip("torch")
+    sp = pytest.importorskip("scipy.sparse")
+    rng = np.random.default_rng(n + sets)
+    rows, cols = [np.arange(n)], [np.arange(n)]
+    for shift in (1, 2, 77, 4999):
+        i = np.flatnonzero(rng.random(n - shift) < 0.7)
+        rows.append(i + shift)
+        cols.append(i)
+    m = sp.csc_matrix((np.ones(sum(map(len, rows))), (np.concatenate(rows), np.concatenate(cols))), (n, n))
+    m.sort_indices()
+    v, p = rng.standard_normal((sets, m.nnz)), rng.standard_normal((sets, n))
+    q = torch.full((sets, n), np.nan, dtype=torch.float64, device="cuda")
+    solver = native.SparseSolver(n, m.indptr.astype(np.int64), m.indices.astype(np.int32), True, sets)
+    solver.multiply(torch.from_numpy(v).cuda(), torch.from_numpy(p).cuda(), q)
+    q = q.cpu().numpy()
+    for s in range(sets):
+        m.data[:] = v[s]
+        A = m + sp.tril(m, -1).T
+        assert np.all(np.abs(q[s] - A @ p[s]) <= 2 * 9 * 2.0 ** -53 * (abs(A) @ np.abs(p[s])))
+
+
 @pytest.mark.parametrize("method,block", [(native.SOLVER_CG, 1), (native.SOLVER_BICGSTAB, 1),
                                           (native.SOLVER_BICGSTAB, 2), (native.SOLVER_BICGSTAB, 4)])
 @pytest.mark.parametrize("n,sets", [(4, 1), (36, 2), (36, 7), (400, 4), (400, 40), (20, 256)])
