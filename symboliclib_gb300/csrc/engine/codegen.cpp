@@ -76,7 +76,7 @@ struct Call {
 //   Strided items (grouped == nullptr): symgbBody<k><L2, ORDER>(..., i, s)
 //     evaluates one work item (instance i, value set s) and loads its own index
 //     and constant entries; ORDER is what it does between these loads, which
-//     no kernel writes, and its first read of x (launchOrder).
+//     no kernel writes, and its first read of x (emitPrologue).
 //   Grouped items: symgbGroup<k><L2, IT, FULL>(..., g, s) evaluates the IT
 //     consecutive instances g*IT .. g*IT+IT-1 of value set s; each index and
 //     constant row is read with one vector load from the padded copies of the
@@ -691,34 +691,19 @@ std::string launchBounds(int tpb, int minBlocks) {
     return s + ")";
 }
 
-// How a launch stands to the one before it (programmatic dependent launch).
-// A launch of another dependency level than its predecessor's waits for it
-// before its first read of x.  Launches of one level read nothing of each
-// other's: they let the next one in at once and run side by side, each waiting
-// at its end instead, so that a launch is complete only when all before it
-// are and the next level's wait covers the whole level.  Cloth 64 x 64, one
-// set (18 kernels, 17 of them of one level, 12 to 9000 instances each): 75.6 us
-// one after another, 58.8 so, of which 47 are the host's launches; 100 x 100, 64
-// sets: 2.10 -> 2.03 ms.
-struct LaunchOrder {
-    bool waitFirst;  // before the first read of x
-    bool letInFirst;  // the next launch may start beside this one
-};
-
-// Prologue of a launch.  One work item per thread (strided): the wait goes
-// behind the table loads of the body, which nothing writes (template argument
-// `order`), and the tables arrive while the predecessor drains.
-int emitPrologue(std::ostringstream& os, const LaunchOrder& o, bool inBody) {
-    const int order = (o.waitFirst ? 1 : 0) | (o.letInFirst ? 2 : 0);
-    if (inBody) return order;
-    if (order) os << "    x = symgbOrder<" << order << ">(x);\n";
+// Every launch waits for its predecessor before its first read of x
+// (programmatic dependent launch): only the wait of the reading grid itself makes
+// earlier grids' writes visible to it.  It lets the next one in when its
+// own work is done.  One work item per thread (strided): the wait goes behind
+// the table loads of the body, which nothing writes (template argument ORDER),
+// and the tables arrive while the predecessor drains.  Returns that argument.
+int emitPrologue(std::ostringstream& os, bool inBody) {
+    if (inBody) return 1;
+    os << "    x = symgbOrder<1>(x);\n";
     return 0;
 }
 
-void emitEpilogue(std::ostringstream& os, const LaunchOrder& o) {
-    if (!o.letInFirst) os << "    symgbLaunchDependents();\n";
-    if (!o.waitFirst) os << "    symgbDependencyWait();\n";
-}
+void emitEpilogue(std::ostringstream& os) { os << "    symgbLaunchDependents();\n"; }
 
 }  // namespace
 
@@ -834,26 +819,20 @@ JitSource generateModule(const std::vector<symgb_kernel_desc>& descs, int numLev
         if (descs[k].num_instances) byLevel[L].push_back((int)k);
     }
     if (cfg.kind == JIT_PLAIN) {
-        std::vector<int> ks;
-        for (std::size_t k = 0; k < descs.size(); ++k)
-            if (descs[k].num_instances * S) ks.push_back((int)k);
-        for (std::size_t q = 0; q < ks.size(); ++q) {
-            const int k = ks[q], level = descs[k].level;
+        for (int k = 0; k < (int)descs.size(); ++k) {
+            if (!(descs[k].num_instances * S)) continue;
             const int tpb = cfg.kernelTpb.at(k);
             const int items = checkedItems(cfg.kernelItems.at(k));
             const std::string name = "symgb_k" + std::to_string(k);
-            const LaunchOrder o{q == 0 || descs[ks[q - 1]].level != level,
-                                q + 1 < ks.size() && descs[ks[q + 1]].level == level};
             os << "extern \"C\" __global__ void " << launchBounds(tpb, cfg.minBlocks) << " " << name << params << ") {\n";
-            const int order = emitPrologue(os, o, items == 1 && !grouped);
+            const int order = emitPrologue(os, items == 1 && !grouped);
             os << "    const unsigned long long b = blockIdx.x;\n";
             emitDispatch(os, {k}, descs, calls, S, tpb, items, 0, "    ", grouped, order);
-            emitEpilogue(os, o);
+            emitEpilogue(os);
             os << "}\n\n";
             out.launches.push_back({name, k, -1, blocksOf({k}, descs, calls, S, tpb, items, grouped), tpb, items, false});
         }
     } else if (cfg.kind == JIT_LEVELS) {
-        const LaunchOrder o{true, false};
         for (int L = 0; L < numLevels; ++L) {
             std::vector<int> ks = byLevel[L];
             if (ks.empty()) continue;
@@ -864,10 +843,10 @@ JitSource generateModule(const std::vector<symgb_kernel_desc>& descs, int numLev
             const int items = checkedItems(cfg.levelItems.at(L));
             const std::string name = "symgb_l" + std::to_string(L);
             os << "extern \"C\" __global__ void " << launchBounds(tpb, cfg.minBlocks) << " " << name << params << ") {\n";
-            const int order = emitPrologue(os, o, items == 1 && !grouped);
+            const int order = emitPrologue(os, items == 1 && !grouped);
             os << "    const unsigned long long b = blockIdx.x;\n";
             emitDispatch(os, ks, descs, calls, S, tpb, items, 0, "    ", grouped, order);
-            emitEpilogue(os, o);
+            emitEpilogue(os);
             os << "}\n\n";
             out.launches.push_back({name, -1, L, blocksOf(ks, descs, calls, S, tpb, items, grouped), tpb, items, false});
         }

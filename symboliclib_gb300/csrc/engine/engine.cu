@@ -455,9 +455,9 @@ int getModule(symgb_unit* u, int kind, std::shared_ptr<const JitModule>* out, do
 
 // Enqueues one evaluation with the compiled executor.  Launches after the
 // first overlap their start-up with the previous launch (programmatic
-// dependent launch; a level's first kernel waits for its predecessor before
-// reading x, the level's others run beside it); with `chainFirst` the first
-// launch's too with whatever is before it on the stream.
+// dependent launch; each kernel waits for its predecessor before reading x);
+// with `chainFirst` the first launch's too with whatever is before it on the
+// stream.
 // With `kernelEvents`, runs the plain module without that overlap and
 // records an event before and after each kernel's launch.
 int enqueueCompiled(symgb_unit* u, const std::vector<cudaEvent_t>* kernelEvents, bool chainFirst) {

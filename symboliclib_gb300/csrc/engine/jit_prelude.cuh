@@ -199,12 +199,11 @@ __device__ bool symgbGridBarrier(B* bar, int* hostError, unsigned long long time
 // this one has issued it or ended.
 __device__ __forceinline__ void symgbDependencyWait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void symgbLaunchDependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-// ORDER & 1: wait, with x passing through the wait so that no read of x can
-// move above it; ORDER & 2: let the next kernel in.
+// ORDER = 1: wait, with x passing through the wait so that no read of x can
+// move above it.
 #define SYMGB_ORDERED
 template <int ORDER>
 __device__ __forceinline__ const double* symgbOrder(const double* x) {
-    if (ORDER & 1) asm volatile("griddepcontrol.wait;" : "+l"(x) : : "memory");
-    if (ORDER & 2) symgbLaunchDependents();
+    if (ORDER) asm volatile("griddepcontrol.wait;" : "+l"(x) : : "memory");
     return x;
 }

@@ -1,0 +1,49 @@
+"""Order of the compiled executor's launches.
+
+A launch reads what earlier launches wrote.  Its own griddepcontrol.wait is
+what makes those writes visible to it, so every generated kernel waits before
+its first read of x, whatever the dependency levels of its neighbours."""
+import functools
+import re
+
+import pytest
+
+from symboliclib_gb300 import native
+
+PLAIN, LEVELS, PERSISTENT = native.SCHEDULE_PLAIN, native.SCHEDULE_LEVELS, native.SCHEDULE_PERSISTENT
+
+
+@functools.lru_cache(None)
+def workload(name, size):
+    return native.Workload(name, size, 8)
+
+
+def entries(src):
+    """Name and body text of every kernel of a generated module."""
+    for m in re.finditer(r'extern "C" __global__ void __launch_bounds__\([^)]*\) (\w+)\(.*?\n}\n', src, re.S):
+        yield m.group(1), m.group(0)[m.group(0).index("{"):]
+
+
+@pytest.mark.parametrize("kind", [PLAIN, LEVELS, PERSISTENT])
+@pytest.mark.parametrize("items,layout", [(1, native.ITEMS_STRIDED), (4, native.ITEMS_STRIDED), (2, native.ITEMS_GROUPED)])
+@pytest.mark.parametrize("name,size,sets", [("cloth", 8, 1), ("cloth", 20, 64), ("ata", 9, 1), ("cotan", 8, 1),
+                                            ("neohookean", 2, 3)])
+def test_every_launch_waits_before_it_reads(name, size, sets, items, layout, kind):
+    u = native.Unit.from_workload(workload(name, size), init=False)
+    u.set_num_sets(sets)
+    native.check(u._lib.symgb_set_item_layout(u.handle, layout))
+    u.set_schedule(kind=kind, items_per_thread=items)
+    src = u.compiled_source(kind)
+    waits = re.search(r"template <int ORDER>.*?symgbOrder.*?\n}", src, re.S).group(0)
+    assert re.search(r"if \(ORDER(?: & 1)?\) asm volatile\(\"griddepcontrol.wait;\" : \"\+l\"\(x\)", waits)
+    found = 0
+    for kernel, body in entries(src):
+        calls = list(re.finditer(r"symgb(?:Body|Mixed|Part|Group)\d+(?:_\d+)?<([^>]*)>\(", body))
+        assert calls, kernel
+        first = body[:calls[0].start()]
+        before = "x = symgbOrder<1>(x);" in first or "symgbDependencyWait();" in first
+        for c in calls:
+            inside = "Group" not in c.group(0) and int((c.group(1) + ", 0").split(",")[1]) & 1
+            assert before or inside, (kernel, c.group(0))
+        found += 1
+    assert found
