@@ -720,6 +720,50 @@ GroupedTables groupedTables(const std::vector<symgb_kernel_desc>& descs) {
     return t;
 }
 
+std::vector<char> besideEarlier(const std::vector<symgb_kernel_desc>& descs, const std::uint32_t* index,
+                                const std::vector<std::uint64_t>& readLo, const std::vector<std::uint64_t>& readHi) {
+    using Range = std::pair<std::uint64_t, std::uint64_t>;  // [first, second)
+    auto writes = [&](std::size_t k) {
+        const symgb_kernel_desc& d = descs[k];
+        return Range(d.output_offset, d.output_offset + d.num_instances * d.num_output_rows);
+    };
+    auto overlap = [](const Range& a, const Range& b) { return std::max(a.first, b.first) < std::min(a.second, b.second); };
+    // The bounds of a kernel's reads settle it for plans in memory order; the
+    // table is only searched where they reach into `r`.
+    auto readsFrom = [&](std::size_t k, const Range& r) {
+        if (readLo[k] > readHi[k] || !overlap(Range(readLo[k], readHi[k] + 1), r)) return false;
+        const symgb_kernel_desc& d = descs[k];
+        for (std::uint32_t a = 0; a < d.num_access; ++a) {
+            const std::uint32_t* row = index + d.index_offset + (std::uint64_t)d.access[2 * a] * d.num_instances;
+            const long long offset = d.access[2 * a + 1];
+            for (std::uint64_t i = 0; i < d.num_instances; ++i) {
+                const std::uint64_t slot = (std::uint64_t)((long long)row[i] + offset);
+                if (slot >= r.first && slot < r.second) return true;
+            }
+        }
+        return false;
+    };
+    std::vector<char> beside(descs.size(), 0);
+    std::vector<std::size_t> group;
+    std::vector<Range> written;  // by the group, adjoining ranges merged
+    for (std::size_t k = 0; k < descs.size(); ++k) {
+        if (!descs[k].num_instances) continue;
+        const Range w = writes(k);
+        bool free = !group.empty();
+        for (std::size_t j = 0; j < written.size() && free; ++j) free = !overlap(w, written[j]) && !readsFrom(k, written[j]);
+        for (std::size_t j = 0; j < group.size() && free; ++j) free = !readsFrom(group[j], w);
+        if (!free) {
+            group.clear();
+            written.clear();
+        }
+        beside[k] = free;
+        group.push_back(k);
+        if (!written.empty() && written.back().second == w.first) written.back().second = w.second;
+        else written.push_back(w);
+    }
+    return beside;
+}
+
 JitSource generateModule(const std::vector<symgb_kernel_desc>& descs, int numLevels, const JitConfig& cfg) {
     JitSource out;
     std::ostringstream os;

@@ -72,6 +72,14 @@ struct JitSource {
 // std::runtime_error for templates it cannot express).
 JitSource generateModule(const std::vector<symgb_kernel_desc>& descs, int numLevels, const JitConfig& cfg);
 
+// Which kernels of a plan may run beside those in front of them, in plan order
+// (JIT_PLAIN): [k] is true where kernel k and the kernels back to the last one
+// with false neither read nor write a slot that another of them writes.
+// From the tables alone, so that a plan's level numbers need not be right.
+// readLo[k], readHi[k]: least and greatest slot kernel k reads (lo > hi: none).
+std::vector<char> besideEarlier(const std::vector<symgb_kernel_desc>& descs, const std::uint32_t* index,
+                                const std::vector<std::uint64_t>& readLo, const std::vector<std::uint64_t>& readHi);
+
 // A compiled and loaded module (jit.cu).  `kernels[j]` is the cudaKernel_t
 // of launches[j], stored as void* (the form the runtime's launch calls take).
 struct JitModule {

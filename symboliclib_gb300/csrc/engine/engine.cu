@@ -453,14 +453,73 @@ int getModule(symgb_unit* u, int kind, std::shared_ptr<const JitModule>* out, do
     return SYMGB_OK;
 }
 
+// The launches of a plain run as branches of the graph being captured: kernels
+// that may run beside each other (besideEarlier) are dealt to kBranches chains,
+// the first of each depending on every chain's end before the group, the others
+// on the one before them in their chain; a launch that depends on one other
+// overlaps its start with it, as in a stream.  Every read is so behind a wait
+// for what wrote it.  Chains, GB300, us a
+// run: one (all launches in order) / two / four / six / one per kernel: cloth
+// 64 x 64 59.4 / 49.2 / 45.2 / 42.8 / 47.4; 100 x 100 x 64 1637 / 1591 / 1579 / 1569 /
+// 1570; A^T A + A 100 from host arrays 65.8 / 62.9 / 62.8 / 62.7 / 66.6.
+class Branches {
+public:
+    explicit Branches(cudaStream_t st) : st_(st) {}
+    // Before a launch; `beside`: beside those since the last one that was not.
+    cudaError_t before(bool beside) {
+        if (!beside) {
+            from_ = std::move(ends_);
+            ends_.clear();
+            count_ = 0;
+        }
+        std::vector<cudaGraphNode_t> deps = from_;
+        if (count_ >= kBranches) deps.assign(1, ends_[count_ % kBranches]);
+        cudaGraphEdgeData edge{};
+        if (deps.size() == 1) {
+            edge.from_port = cudaGraphKernelNodePortProgrammatic;
+            edge.type = cudaGraphDependencyTypeProgrammatic;
+        }
+        return set(deps, edge);
+    }
+    // After it.
+    cudaError_t after() {
+        cudaStreamCaptureStatus status;
+        const cudaGraphNode_t* deps = nullptr;
+        const cudaGraphEdgeData* edges = nullptr;
+        std::size_t n = 0;
+        const cudaError_t e = cudaStreamGetCaptureInfo(st_, &status, nullptr, nullptr, &deps, &edges, &n);
+        if (e != cudaSuccess) return e;
+        if (n != 1) return cudaErrorStreamCaptureUnjoined;
+        if (count_ < kBranches) ends_.push_back(deps[0]);
+        else ends_[count_ % kBranches] = deps[0];
+        ++count_;
+        return cudaSuccess;
+    }
+    // What follows depends on every branch.
+    cudaError_t join() { return set(ends_, cudaGraphEdgeData{}); }
+
+private:
+    static constexpr std::size_t kBranches = 6;
+    cudaError_t set(std::vector<cudaGraphNode_t>& deps, const cudaGraphEdgeData& edge) {
+        std::vector<cudaGraphEdgeData> edges(deps.size(), edge);
+        return cudaStreamUpdateCaptureDependencies(st_, deps.empty() ? nullptr : deps.data(),
+                                                   deps.empty() ? nullptr : edges.data(), deps.size(),
+                                                   cudaStreamSetCaptureDependencies);
+    }
+    cudaStream_t st_;
+    std::vector<cudaGraphNode_t> from_, ends_;  // what the group depends on; the branches' ends
+    std::size_t count_ = 0;                     // launches of the group
+};
+
 // Enqueues one evaluation with the compiled executor.  Launches after the
 // first overlap their start-up with the previous launch (programmatic
 // dependent launch; each kernel waits for its predecessor before reading x);
 // with `chainFirst` the first launch's too with whatever is before it on the
-// stream.
+// stream.  With `branches` (in a capture of the unit's own) a plain run's
+// independent kernels become branches of the graph.
 // With `kernelEvents`, runs the plain module without that overlap and
 // records an event before and after each kernel's launch.
-int enqueueCompiled(symgb_unit* u, const std::vector<cudaEvent_t>* kernelEvents, bool chainFirst) {
+int enqueueCompiled(symgb_unit* u, const std::vector<cudaEvent_t>* kernelEvents, bool chainFirst, Branches* branches) {
     std::shared_ptr<const JitModule> m;
     if (kernelEvents) {
         if (int e = getModule(u, SYMGB_SCHEDULE_PLAIN, &m)) return e;
@@ -497,7 +556,9 @@ int enqueueCompiled(symgb_unit* u, const std::vector<cudaEvent_t>* kernelEvents,
             at[na].val.cooperative = 1;
             ++na;
         }
-        if (j > 0 ? !kernelEvents : chainFirst && !L.cooperative) {
+        if (branches) {
+            SYMGB_CUDA(branches->before(u->beside[L.kernel]));
+        } else if (j > 0 ? !kernelEvents : chainFirst && !L.cooperative) {
             at[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
             at[na].val.programmaticStreamSerializationAllowed = 1;
             ++na;
@@ -512,8 +573,10 @@ int enqueueCompiled(symgb_unit* u, const std::vector<cudaEvent_t>* kernelEvents,
         if (kernelEvents && L.kernel >= 0) SYMGB_CUDA(cudaEventRecord((*kernelEvents)[2 * L.kernel], u->stream));
         SYMGB_CUDA(cudaLaunchKernelExC(&cfg, m->kernels[j], args));
         if (kernelEvents && L.kernel >= 0) SYMGB_CUDA(cudaEventRecord((*kernelEvents)[2 * L.kernel + 1], u->stream));
+        if (branches) SYMGB_CUDA(branches->after());
         ++launches;
     }
+    if (branches) SYMGB_CUDA(branches->join());
     u->launchesPerRun = launches;
     u->lastRunDirect = m->direct;
     return SYMGB_OK;
@@ -522,8 +585,10 @@ int enqueueCompiled(symgb_unit* u, const std::vector<cudaEvent_t>* kernelEvents,
 // Enqueues one evaluation on the unit's stream.  With `kernelEvents`, runs the
 // plain schedule whatever the unit's and records an event before and after
 // each kernel's launch (per-kernel timing).
-int enqueueRun(symgb_unit* u, const std::vector<cudaEvent_t>* kernelEvents = nullptr, bool chainFirst = false) {
-    if (u->compiledExec()) return enqueueCompiled(u, kernelEvents, chainFirst);
+int enqueueRun(symgb_unit* u, const std::vector<cudaEvent_t>* kernelEvents = nullptr, bool chainFirst = false,
+               Branches* branches = nullptr) {
+    if (u->compiledExec())
+        return enqueueCompiled(u, kernelEvents, chainFirst, u->sched.kind == SYMGB_SCHEDULE_PLAIN ? branches : nullptr);
     u->lastRunDirect = false;
     if (int e = buildTiles(u)) return e;
     const int items = u->items();
@@ -682,7 +747,8 @@ int runAsync(symgb_unit* u) {
             cudaError_t ce = cudaStreamBeginCapture(u->stream, cudaStreamCaptureModeThreadLocal);
             int e = SYMGB_OK;
             if (ce == cudaSuccess) {
-                e = enqueueRun(u);
+                Branches branches(u->stream);
+                e = enqueueRun(u, nullptr, false, &branches);
                 ce = cudaStreamEndCapture(u->stream, &g);
             }
             u->stream = saved;
@@ -788,24 +854,42 @@ int symgb_init(symgb_unit_t u, const uint32_t* index_data, const uint32_t* out_i
     // bounds checks.  The slots some kernel reads are noted for the direct
     // result plan.
     std::vector<std::uint8_t> slotRead(u->numTotalMemory, 0);
+    std::vector<symgb_kernel_desc> descs;
+    std::vector<std::uint64_t> readLo, readHi;
     for (const auto& k : u->kernels) {
         const auto& d = k.desc;
-        for (std::uint32_t a = 0; a < d.num_access; ++a) {
+        const std::uint64_t n = d.num_instances;
+        std::uint64_t lo = ~0ull, hi = 0;
+        std::map<std::uint32_t, std::pair<std::uint32_t, std::uint32_t>> bounds;  // of a row's entries
+        for (std::uint32_t a = 0; a < d.num_access && n; ++a) {
             const std::uint32_t row = (std::uint32_t)k.access[2 * a];
             const long long off = k.access[2 * a + 1];
-            const std::uint32_t* pr = index_data + d.index_offset + (std::uint64_t)row * d.num_instances;
-            for (std::uint64_t i = 0; i < d.num_instances; ++i) {
-                const long long slot = (long long)pr[i] + off;
-                if (slot < 0 || (std::uint64_t)slot >= u->numTotalMemory)
-                    return fail(SYMGB_ERR_ARGUMENT, "index table entry outside x");
-                slotRead[(std::size_t)slot] = 1;
+            const std::uint32_t* pr = index_data + d.index_offset + (std::uint64_t)row * n;
+            auto b = bounds.find(row);
+            if (b == bounds.end()) {
+                std::uint32_t least = pr[0], most = pr[0];
+                for (std::uint64_t i = 1; i < n; ++i) {
+                    least = std::min(least, pr[i]);
+                    most = std::max(most, pr[i]);
+                }
+                b = bounds.emplace(row, std::make_pair(least, most)).first;
             }
+            const long long first = (long long)b->second.first + off, last = (long long)b->second.second + off;
+            if (first < 0 || (std::uint64_t)last >= u->numTotalMemory)
+                return fail(SYMGB_ERR_ARGUMENT, "index table entry outside x");
+            lo = std::min(lo, (std::uint64_t)first);
+            hi = std::max(hi, (std::uint64_t)last);
+            for (std::uint64_t i = 0; i < n; ++i) slotRead[(std::size_t)((long long)pr[i] + off)] = 1;
         }
+        descs.push_back(d);
+        readLo.push_back(lo);
+        readHi.push_back(hi);
     }
     for (std::uint64_t j = 0; j < u->numOutputValues; ++j)
         if (out_index_data[j] >= u->numTotalMemory) return fail(SYMGB_ERR_ARGUMENT, "output id outside x");
     u->release();
     u->jitModules.clear();  // their direct result rows belong to the previous tables
+    u->beside = symgb::engine::besideEarlier(descs, index_data, readLo, readHi);
     // Direct result plan: an output row is direct when each of its slots is
     // read by no kernel and is the slot of exactly one result position
     // (positions are 32-bit in the table: larger result sets are gathered).

@@ -130,6 +130,8 @@ struct symgb_unit {
     // One run as a graph (runAsync), until the configuration changes:
     // graphDirect is lastRunDirect after it, ranBefore whether the configuration
     // has run launch by launch.
+    // `beside`: kernels that may run beside earlier ones (besideEarlier).
+    std::vector<char> beside;
     cudaGraphExec_t graph = nullptr;
     bool graphValid = false, graphDirect = false, ranBefore = false;
     // Compiled executor: modules by configuration key (schedule kind, math,

@@ -2,13 +2,20 @@
 
 A launch reads what earlier launches wrote.  Its own griddepcontrol.wait is
 what makes those writes visible to it, so every generated kernel waits before
-its first read of x, whatever the dependency levels of its neighbours."""
+its first read of x, whatever the dependency levels of its neighbours.  Launches
+that a replayed plain run puts side by side are chosen from what the tables make
+them read and write, not from the plan's level numbers."""
 import functools
 import re
+import subprocess
 
+import numpy as np
 import pytest
 
-from symboliclib_gb300 import native
+from conftest import ROOT
+from symboliclib_gb300 import build, native
+
+import oracle.cpu as ocpu
 
 PLAIN, LEVELS, PERSISTENT = native.SCHEDULE_PLAIN, native.SCHEDULE_LEVELS, native.SCHEDULE_PERSISTENT
 
@@ -47,3 +54,36 @@ def test_every_launch_waits_before_it_reads(name, size, sets, items, layout, kin
             assert before or inside, (kernel, c.group(0))
         found += 1
     assert found
+
+
+def test_side_by_side_kernels_share_no_written_slot():
+    out, lib = build.OBJ / "beside_earlier_test", build.LIB
+    subprocess.run(["g++", "-std=c++17", "-O1", f"-I{ROOT / 'include'}", f"-I{build.CSRC / 'engine'}",
+                    str(ROOT / "tests" / "cpp" / "beside_earlier.cpp"), "-o", str(out), f"-L{lib}", "-lsymgb",
+                    f"-Wl,-rpath,{lib}"], check=True, capture_output=True, text=True)
+    r = subprocess.run([str(out)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("careless", [False, True])
+@pytest.mark.parametrize("name,size", [("cotan", 8), ("cloth", 12), ("ata", 9), ("neohookean", 2)])
+def test_plain_runs_need_no_levels(name, size, careless):
+    """Plain runs evaluate the kernels in plan order, also when every kernel
+    claims the same level: the first run launch by launch, the others replayed."""
+    w = native.Workload(name, size, 5)
+    rng = np.random.default_rng(size)
+    runs = []
+    for _ in range(4):
+        ins = [a * (1 + 1e-3 * rng.uniform(-1, 1, a.size)) for a in w.inputs]
+        runs.append((ins, ocpu.evaluate(w.plan, w.index_data, w.out_index_data, w.const_data, ins)[0]))
+    if careless:
+        for k in range(w.plan.contents.num_kernels):
+            w.plan.contents.kernels[k].level = 0
+    u = native.Unit.from_workload(w)
+    u.set_schedule(kind=PLAIN, math=native.MATH_EXACT)
+    for ins, ref in runs:
+        for i, a in enumerate(ins):
+            u.set_arg(i, a)
+        u.run()
+        assert np.array_equal(u.get_result(0).view(np.uint64), ref.view(np.uint64))
