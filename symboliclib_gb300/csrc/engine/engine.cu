@@ -12,6 +12,7 @@
 // blocks cover consecutive work items, so for S >= 32 a warp shares one
 // instance and its index loads are broadcasts, and for S = 1 a warp covers 32
 // consecutive instances and its index loads are one coalesced 128-byte line.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -203,15 +204,32 @@ cudaError_t copyChained(const symgb_unit* u, const double* src, double* dst, std
     return n ? launchChained(u, copyKernel, dim3((unsigned)((n + 2047) / 2048)), src, dst, n) : cudaSuccess;
 }
 
-// Memory of the unit's device, for the copy kernel; other memory takes the
-// runtime's copies.
-bool onDevice(const symgb_unit* u, const void* p) {
+// Whether the copy kernel may take the `n` doubles at `p`: memory of the unit's
+// device, all in one allocation, aligned.  Anything else takes the runtime's
+// copies, which copy from any alignment and other memory, and refuse what an
+// allocation does not hold where a kernel would fault.
+bool onDevice(const symgb_unit* u, const double* p, std::uint64_t n) {
+    if ((std::uintptr_t)p % alignof(double)) return false;
     cudaPointerAttributes a;
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    return a.type == cudaMemoryTypeDevice && a.device == u->device;
+    if (a.type != cudaMemoryTypeDevice || a.device != u->device) return false;
+    using AddressRange = CUresult (*)(CUdeviceptr*, std::size_t*, CUdeviceptr);
+    static const AddressRange addressRange = [] {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &fn, 3020, cudaEnableDefault, &found) != cudaSuccess) {
+            cudaGetLastError();
+            fn = nullptr;
+        }
+        return (AddressRange)fn;
+    }();
+    CUdeviceptr base = 0;
+    std::size_t size = 0;
+    if (!addressRange || addressRange(&base, &size, (CUdeviceptr)p) != CUDA_SUCCESS) return false;
+    return n * sizeof(double) <= size - (std::size_t)((CUdeviceptr)p - base);
 }
 
 }  // namespace
@@ -1019,7 +1037,7 @@ int symgb_get_result_sets_device(symgb_unit_t u, double* d, int k) {
     int err = SYMGB_OK;
     if (resultsInRes(u, &err)) {
         if (err) return err;
-        if (onDevice(u, d))
+        if (onDevice(u, d, u->outLength[k]))
             SYMGB_CUDA(copyChained(u, u->res.ptr + u->outStart[k], d, u->outLength[k]));
         else if (u->outLength[k])
             SYMGB_CUDA(cudaMemcpyAsync(d, u->res.ptr + u->outStart[k], u->outLength[k] * 8, cudaMemcpyDefault,
@@ -1094,7 +1112,7 @@ int symgb_set_arg_sets_device(symgb_unit_t u, const double* d, int i) {
     if (i < 0 || (std::size_t)i >= u->argStart.size() || !d) return fail(SYMGB_ERR_ARGUMENT, "bad argument index");
     const std::uint64_t len = u->argLength[i];
     if (u->numSets == 1) {
-        if (onDevice(u, d))
+        if (onDevice(u, d, len))
             SYMGB_CUDA(copyChained(u, d, u->x.ptr + u->argStart[i], len));
         else
             SYMGB_CUDA(cudaMemcpyAsync(u->x.ptr + u->argStart[i], d, len * 8, cudaMemcpyDeviceToDevice, u->stream));
