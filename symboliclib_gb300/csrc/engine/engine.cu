@@ -61,10 +61,13 @@ namespace {
 // The copies between a caller's buffers and x or res below are launched with
 // programmatic stream serialisation, as the run's own launches are (chained):
 // each waits for its predecessor before it touches memory and lets the next
-// one in when it is done.  A boundary between two such kernels costs about 1 us
-// of the stream; one with a copy operation or without the attribute 2 to 4 (cotan
-// 100 x 100, inputs and results on the device: 18.4 us with copy operations and an
-// unchained first launch, 12.2 so).
+// one in when it is done.  What the predecessor may have written is read with
+// ordinary loads: the read-only path (__ldg) is for what does not change while
+// a kernel is resident, and these are resident before their predecessor ends.
+// A boundary between two such kernels costs about 1 us of the stream; one with
+// a copy operation or without the attribute 2 to 4 (cotan 100 x 100, inputs and
+// results on the device: 18.4 us with copy operations and an unchained first
+// launch, 12.2 so).
 
 // dst[q] = src[q]; 16 bytes at a time where both are aligned to it.
 __global__ void __launch_bounds__(256) copyKernel(const double* src, double* dst, std::uint64_t n) {
@@ -89,14 +92,14 @@ __global__ void __launch_bounds__(256) copyKernel(const double* src, double* dst
 }
 
 // x[(start + j) * S + s] = in[s * len + j]
-__global__ void scatterKernel(const double* __restrict__ in, std::uint64_t start, std::uint64_t len, unsigned S,
+__global__ void scatterKernel(const double* in, std::uint64_t start, std::uint64_t len, unsigned S,
                               double* __restrict__ x) {
     const std::uint64_t w = (std::uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     in = symgbOrder<1>(in);
     if (w >= len * S) return;
     const std::uint64_t j = w / S;
     const unsigned s = (unsigned)(w - j * S);
-    x[(start + j) * S + s] = __ldg(in + (std::uint64_t)s * len + j);
+    x[(start + j) * S + s] = in[(std::uint64_t)s * len + j];
     symgbLaunchDependents();
 }
 
@@ -109,7 +112,7 @@ __global__ void scatterKernel(const double* __restrict__ in, std::uint64_t start
 constexpr unsigned kSetTile = 32;
 
 // out[s * len + j] = x[ids[j] * S + s]
-__global__ void __launch_bounds__(256) gatherSetsKernel(const double* __restrict__ x,
+__global__ void __launch_bounds__(256) gatherSetsKernel(const double* x,
                                                         const std::uint32_t* __restrict__ ids, std::uint64_t len,
                                                         unsigned S, double* __restrict__ out) {
     __shared__ double tile[kSetTile][kSetTile + 1];
@@ -119,7 +122,7 @@ __global__ void __launch_bounds__(256) gatherSetsKernel(const double* __restrict
     x = symgbOrder<1>(x);
     for (unsigned p = warp; p < kSetTile; p += 8) {
         const std::uint64_t j = j0 + p;
-        if (j < len && s0 + lane < S) tile[p][lane] = __ldg(x + (std::uint64_t)__ldg(ids + j) * S + s0 + lane);
+        if (j < len && s0 + lane < S) tile[p][lane] = x[(std::uint64_t)__ldg(ids + j) * S + s0 + lane];
     }
     __syncthreads();
     for (unsigned q = warp; q < kSetTile; q += 8) {
@@ -130,7 +133,7 @@ __global__ void __launch_bounds__(256) gatherSetsKernel(const double* __restrict
 }
 
 // x[(start + j) * S + s] = in[s * len + j]
-__global__ void __launch_bounds__(256) scatterSetsKernel(const double* __restrict__ in, std::uint64_t start,
+__global__ void __launch_bounds__(256) scatterSetsKernel(const double* in, std::uint64_t start,
                                                          std::uint64_t len, unsigned S, double* __restrict__ x) {
     __shared__ double tile[kSetTile][kSetTile + 1];
     const std::uint64_t j0 = (std::uint64_t)blockIdx.x * kSetTile;
@@ -139,7 +142,7 @@ __global__ void __launch_bounds__(256) scatterSetsKernel(const double* __restric
     in = symgbOrder<1>(in);
     for (unsigned q = warp; q < kSetTile; q += 8) {
         const std::uint64_t j = j0 + lane;
-        if (s0 + q < S && j < len) tile[lane][q] = __ldg(in + (std::uint64_t)(s0 + q) * len + j);
+        if (s0 + q < S && j < len) tile[lane][q] = in[(std::uint64_t)(s0 + q) * len + j];
     }
     __syncthreads();
     for (unsigned p = warp; p < kSetTile; p += 8) {
@@ -163,11 +166,11 @@ __global__ void padRowsKernel(const T* __restrict__ src, T* __restrict__ dst, st
 
 // res[pos[t]] = x[slot[t]]: the results of the rows that are not written
 // straight into res (one value set).
-__global__ void restGatherKernel(const double* __restrict__ x, const std::uint32_t* __restrict__ pos,
+__global__ void restGatherKernel(const double* x, const std::uint32_t* __restrict__ pos,
                                  const std::uint32_t* __restrict__ slot, std::uint64_t count, double* __restrict__ res) {
     const std::uint64_t t = (std::uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     x = symgbOrder<1>(x);
-    if (t < count) res[__ldg(pos + t)] = __ldg(x + __ldg(slot + t));
+    if (t < count) res[__ldg(pos + t)] = x[__ldg(slot + t)];
     symgbLaunchDependents();
 }
 

@@ -56,6 +56,19 @@ def test_every_launch_waits_before_it_reads(name, size, sets, items, layout, kin
     assert found
 
 
+def test_copy_kernels_read_what_may_change_with_ordinary_loads():
+    """Kernels that start before their predecessor has ended do not read its
+    results through the read-only path."""
+    found = 0
+    for path in (build.CSRC / "engine").glob("*.cu*"):
+        for m in re.finditer(r"__global__ [^;{]*?\((.*?)\) \{(.*?)\n}", path.read_text(), re.S):
+            for p in re.findall(r"symgbOrder<1>\((\w+)\)", m.group(2)):
+                found += 1
+                assert not re.search(rf"__ld\w+\({p}\b", m.group(2)), (path.name, p)
+                assert not re.search(rf"__restrict__ {p}\b", m.group(1)), (path.name, p)
+    assert found >= 5
+
+
 def test_side_by_side_kernels_share_no_written_slot():
     out, lib = build.OBJ / "beside_earlier_test", build.LIB
     subprocess.run(["g++", "-std=c++17", "-O1", f"-I{ROOT / 'include'}", f"-I{build.CSRC / 'engine'}",
