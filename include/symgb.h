@@ -369,7 +369,9 @@ const char* symgb_plan_last_error(void);
  * definite) or BiCGSTAB (any nonsingular A; the cloth matrices of a deformed
  * sheet are indefinite).  It starts from x = 0 and stops once every system's
  * |r| / |b| <= tol (checked every 16 iterations) or after max_iter
- * iterations, reporting both.  symgb_solver_multiply computes q = A p. */
+ * iterations, reporting both.  A system whose residual is not finite (NaN or Inf
+ * in its data, or a breakdown) is not waited for and makes the reported
+ * residual infinite.  symgb_solver_multiply computes q = A p. */
 #define SYMGB_SOLVER_CG 0
 #define SYMGB_SOLVER_BICGSTAB 1
 typedef struct symgb_solver* symgb_solver_t;

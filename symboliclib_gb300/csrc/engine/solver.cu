@@ -32,6 +32,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <limits>
 #include <string>
 #include <vector>
 
@@ -707,6 +708,25 @@ static void product(symgb_solver_t s, const double* z, const double* w, double* 
               : (wide ? launch(spmv<false, true>) : launch(spmv<false, false>));
 }
 
+// Largest |r| / |b| of the S systems from their squares; infinity where one is
+// not finite: NaN or Inf in the data, squares beyond the double range, or a
+// breakdown, none of which an iteration comes back from.  `open`: some other
+// system has not reached `tol`.
+static double worstResidual(const double* rr, const double* bb, unsigned S, double tol, bool* open) {
+    double worst = 0.0;
+    *open = false;
+    for (unsigned k = 0; k < S; ++k) {
+        const double rel = rr[k] == 0.0 ? 0.0 : std::sqrt(rr[k] / bb[k]);
+        if (!std::isfinite(rel) || !std::isfinite(bb[k])) {
+            worst = std::numeric_limits<double>::infinity();
+            continue;
+        }
+        worst = std::max(worst, rel);
+        *open |= !(rel <= tol);
+    }
+    return worst;
+}
+
 int symgb_solver_multiply(symgb_solver_t s, const double* values, const double* p_dev, double* q_dev, void* stream) {
     using symgb::engine::setLastError;
     if (!s || !values || !p_dev || !q_dev) return setLastError(SYMGB_ERR_ARGUMENT, "solver: null argument");
@@ -762,12 +782,9 @@ static int solveCg(symgb_solver_t s, const double* values, const double* b_dev, 
         }
         cudaMemcpyAsync(s->hostScalars, rr, S * sizeof(double), cudaMemcpyDeviceToHost, st);
         if (cudaStreamSynchronize(st) != cudaSuccess) return setLastError(SYMGB_ERR_CUDA, "solver: solve failed");
-        worst = 0.0;
-        for (unsigned k = 0; k < S; ++k) {
-            const double rel = bbHost[k] > 0 ? std::sqrt(s->hostScalars[k] / bbHost[k]) : 0.0;
-            worst = std::max(worst, rel);
-        }
-        if (worst <= tol) break;
+        bool open;
+        worst = worstResidual(s->hostScalars, bbHost.data(), S, tol, &open);
+        if (!open) break;
     }
     transposeSets<<<blocksFor(work), kThreads, 0, st>>>(s->x.ptr, s->n, S, x_dev);
     if (cudaStreamSynchronize(st) != cudaSuccess || cudaGetLastError() != cudaSuccess)
@@ -836,10 +853,9 @@ static int solveBicgstab(symgb_solver_t s, const double* values, const double* b
         }
         cudaMemcpyAsync(s->hostScalars, rr, S * sizeof(double), cudaMemcpyDeviceToHost, st);
         if (cudaStreamSynchronize(st) != cudaSuccess) return setLastError(SYMGB_ERR_CUDA, "solver: solve failed");
-        worst = 0.0;
-        for (unsigned k = 0; k < S; ++k)
-            worst = std::max(worst, bbHost[k] > 0 ? std::sqrt(s->hostScalars[k] / bbHost[k]) : 0.0);
-        if (worst <= tol) break;
+        bool open;
+        worst = worstResidual(s->hostScalars, bbHost.data(), S, tol, &open);
+        if (!open) break;
     }
     transposeSets<<<blocksFor(work), kThreads, 0, st>>>(s->x.ptr, s->n, S, x_dev);
     if (cudaStreamSynchronize(st) != cudaSuccess || cudaGetLastError() != cudaSuccess)

@@ -99,3 +99,35 @@ def test_solve_diagonally_dominant(n, sets, method, block):
         for s in {0, sets - 1}:
             ref = np.linalg.solve(dense(n, cp, ri, v[s], True), b[s])
             assert np.linalg.norm(x[s].cpu().numpy() - ref) <= 1e-11 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("method", [native.SOLVER_CG, native.SOLVER_BICGSTAB])
+@pytest.mark.parametrize("where", ["b nan", "b inf", "values nan", "b huge", "all"])
+def test_systems_that_are_not_finite_are_not_reported_as_solved(method, where):
+    """Beside them the other systems, one of them with b = 0, are solved to the
+    tolerance, and nobody waits for what cannot converge."""
+    torch = pytest.importorskip("torch")
+    n, sets = 60, 5
+    rng = np.random.default_rng(4)
+    cp, ri = pattern(n, 0.1, True, rng)
+    col = np.repeat(np.arange(n), np.diff(cp))
+    v = rng.uniform(-1.0, 1.0, (sets, len(ri))) * 0.02
+    v[:, ri == col] = rng.uniform(1.0, 3.0, (sets, n))
+    b = rng.standard_normal((sets, n))
+    b[3] = 0.0
+    bad = list(range(sets)) if where == "all" else [1]
+    for s in bad:
+        if where == "values nan":
+            v[s, 7] = np.nan
+        elif where == "b huge":
+            b[s] *= 1e200  # its square is beyond the double range
+        else:
+            b[s, 5] = np.inf if where == "b inf" else np.nan
+    solver = native.SparseSolver(n, cp, ri, True, sets)
+    x = torch.full((sets, n), 7.0, dtype=torch.float64, device="cuda")
+    it, res = solver.solve(torch.from_numpy(v).cuda(), torch.from_numpy(b).cuda(), x, tol=1e-12, max_iter=640,
+                           method=method)
+    assert res == np.inf and it <= 64
+    for s in set(range(sets)) - set(bad):
+        ref = np.linalg.solve(dense(n, cp, ri, v[s], True), b[s])
+        assert np.linalg.norm(x[s].cpu().numpy() - ref) <= 1e-11 * np.linalg.norm(ref)
