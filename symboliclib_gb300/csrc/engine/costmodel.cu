@@ -309,8 +309,6 @@ int pass(symgb_mlp* net, int n, const float* y, bool backward) {
     if (sizeof(float) * std::max(net->in * h, h * h) > kLayerBytes)
         return mlpFail(SYMGB_ERR_CUDA, "MLP layer exceeds 48 KB of weights");
     const std::size_t smem = L.sharedBytes();
-    if (smem > 48 * 1024)
-        MLP_CUDA(cudaFuncSetAttribute(tilePass, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     tilePass<<<passBlocks(net, n), kThreads, smem>>>(net->X, y, net->params, n, L, net->out, net->sq,
                                                      backward ? net->parts : nullptr);
     return SYMGB_OK;
@@ -374,6 +372,12 @@ int symgb_mlp_create(int inputs, int hidden, unsigned long long seed, symgb_mlp_
     int device = 0;
     MLP_CUDA(cudaGetDevice(&device));
     MLP_CUDA(cudaDeviceGetAttribute(&net->smCount, cudaDevAttrMultiProcessorCount, device));
+    // The shared memory a pass may have is the kernel's, not the network's: the
+    // most there is, as another thread's network could lower a size of this
+    // one's own between here and its launch.
+    int most = 0;
+    MLP_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+    MLP_CUDA(cudaFuncSetAttribute(tilePass, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     *out = net.release();
     return SYMGB_OK;
 }

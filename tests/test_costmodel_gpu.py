@@ -1,6 +1,8 @@
 """The cost model's kernels at the edges of their tiles (16 samples, 4 rows and
 samples per thread, two blocks per SM), against the float64 restatement
 (oracle/mlp.py)."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -34,3 +36,25 @@ def test_layers_beyond_a_blocks_share_are_refused():
     net = native.MLP(4, 128, seed=1)  # 128 x 128 weights: 64 KB
     with pytest.raises(RuntimeError):
         net.predict(np.zeros((8, 4), np.float32))
+
+
+def test_networks_of_several_sizes_on_several_threads():
+    """The shared memory that a launch may have is a property of the kernel, not
+    of the network."""
+    def work(inputs, hidden, out):
+        rng = np.random.default_rng(inputs)
+        X, y = rng.standard_normal((40, inputs)).astype(np.float32), rng.standard_normal(40).astype(np.float32)
+        try:
+            net = native.MLP(inputs, hidden, seed=3)
+            first = net.gradient(X, y)[0]
+            out.append(all(np.array_equal(net.gradient(X, y)[0], first) for _ in range(400)))
+        except RuntimeError as e:
+            out.append(str(e))
+    results = [[] for _ in range(4)]
+    threads = [threading.Thread(target=work, args=(*shape, out))
+               for shape, out in zip([(50, 64), (111, 110), (256, 48), (20, 96)], results)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert results == [[True]] * 4
