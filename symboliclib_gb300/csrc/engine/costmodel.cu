@@ -143,9 +143,9 @@ __global__ void __launch_bounds__(kThreads) tilePass(const float* __restrict__ X
     const int tiles = (n + kTile - 1) / kTile;
     for (int t = blockIdx.x; t < tiles; t += gridDim.x, add = true) {
         const int row0 = t * kTile, rows = min(kTile, n - row0);
-        for (int q = threadIdx.x; q < kTile * in; q += kThreads) {  // past the end: the last row again, its error taken as zero
+        for (int q = threadIdx.x; q < kTile * in; q += kThreads) {  // past the end zeros, their error taken as zero
             const int r = q / in, i = q % in;
-            sX[i * kRow + r] = X[(std::size_t)(row0 + min(r, rows - 1)) * in + i];
+            sX[i * kRow + r] = r < rows ? X[(std::size_t)(row0 + r) * in + i] : 0.f;
         }
         __syncthreads();
         forwardLayer(sX, sW1, h, sb1, sH1, in, h);
@@ -201,7 +201,8 @@ __global__ void __launch_bounds__(kThreads) tilePass(const float* __restrict__ X
     }
 }
 
-// s + e += v, e the rounding error of the running sum (Knuth's TwoSum).
+// s + e += v, e the rounding error of the running sum (Knuth's TwoSum); NaN
+// once the sum is not finite.
 __device__ __forceinline__ void addCompensated(float& s, float& e, float v) {
     const float t = __fadd_rn(s, v), z = __fsub_rn(t, s);
     e = __fadd_rn(e, __fadd_rn(__fsub_rn(s, __fsub_rn(t, z)), __fsub_rn(v, z)));
@@ -234,7 +235,7 @@ __global__ void __launch_bounds__(kThreads) reduceUpdate(const float* __restrict
         addCompensated(s, e, ss[t * 32 + lane]);
         e += se[t * 32 + lane];
     }
-    const float gi = s + e;
+    const float gi = isfinite(s) ? s + e : s;
     if (!p) {
         g[q] = gi;
         return;

@@ -58,3 +58,15 @@ def test_networks_of_several_sizes_on_several_threads():
     for t in threads:
         t.join()
     assert results == [[True]] * 4
+
+
+@pytest.mark.parametrize("n", [16, 17, 40])
+def test_gradients_beyond_the_range_are_infinite(n):
+    """One sample whose activations overflow, in a full tile and in ragged ones:
+    sums with one infinity are infinite, not NaN."""
+    X = np.ones((n, 1), np.float32)
+    X[-1] = 3e38
+    net = native.MLP(1, 1, seed=1)
+    net.set_params(np.array([2, 0, 1, 0, 1, 0], np.float32))  # W1 b1 W2 b2 W3 b3
+    g, loss = net.gradient(X, np.zeros(n, np.float32))
+    assert np.all(g == np.inf) and loss == np.inf
