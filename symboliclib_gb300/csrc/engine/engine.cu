@@ -732,6 +732,39 @@ int enqueueRun(symgb_unit* u, const std::vector<cudaEvent_t>* kernelEvents = nul
     return SYMGB_OK;
 }
 
+// One run in the current configuration as a graph.
+int makeGraph(symgb_unit* u) {
+    // Nothing may be compiled, loaded or allocated during the capture.
+    if (u->compiledExec()) {
+        std::shared_ptr<const JitModule> m;
+        if (int e = getModule(u, u->sched.kind, &m)) return e;
+    } else if (int e = buildTiles(u)) {
+        return e;
+    }
+    const RelaxedCapture relaxed;
+    cudaStream_t saved = u->stream;
+    u->stream = u->ownStream;  // a stream of the caller's may be one that cannot be captured
+    cudaGraph_t g = nullptr;
+    int e = SYMGB_OK;
+    cudaError_t ce = cudaStreamBeginCapture(u->stream, cudaStreamCaptureModeRelaxed);
+    if (ce == cudaSuccess) {
+        Branches branches(u->stream);
+        e = enqueueRun(u, nullptr, false, &branches);
+        ce = cudaStreamEndCapture(u->stream, &g);
+    }
+    u->stream = saved;
+    if (!e && ce != cudaSuccess) e = fail(SYMGB_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(ce));
+    if (!e && (ce = cudaGraphInstantiate(&u->graph, g, 0)) != cudaSuccess) {
+        u->graph = nullptr;
+        e = fail(SYMGB_ERR_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(ce));
+    }
+    if (g) cudaGraphDestroy(g);
+    if (e) return e;
+    u->graphValid = true;
+    u->graphDirect = u->lastRunDirect;
+    return SYMGB_OK;
+}
+
 int runAsync(symgb_unit* u) {
     if (!u->initialized) return fail(SYMGB_ERR_STATE, "run before init");
     // A run that writes its results straight into res waits (on the unit's
@@ -753,35 +786,18 @@ int runAsync(symgb_unit* u) {
     // once does not pay for a graph; nor is one made inside a capture of the
     // caller's, which takes the launches themselves.
     constexpr int kGraphLaunches = 6;
-    const bool graph = u->sched.use_graph || (u->ranBefore && u->launchesPerRun >= kGraphLaunches && !capturing);
-    if (graph) {
-        if (!u->graphValid) {
-            if (u->compiledExec()) {  // nothing may be compiled or loaded during the capture
-                std::shared_ptr<const JitModule> m;
-                if (int e = getModule(u, u->sched.kind, &m)) return e;
-            }
-            if (int e = buildTiles(u)) return e;
-            // smem attributes must be set outside capture
-            cudaGraph_t g;
-            cudaStream_t saved = u->stream;
-            u->stream = u->ownStream;  // a stream of the caller's may be one that cannot be captured
-            cudaError_t ce = cudaStreamBeginCapture(u->stream, cudaStreamCaptureModeThreadLocal);
-            int e = SYMGB_OK;
-            if (ce == cudaSuccess) {
-                Branches branches(u->stream);
-                e = enqueueRun(u, nullptr, false, &branches);
-                ce = cudaStreamEndCapture(u->stream, &g);
-            }
-            u->stream = saved;
-            if (e) return e;
-            if (ce != cudaSuccess) return fail(SYMGB_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(ce));
-            ce = cudaGraphInstantiate(&u->graph, g, 0);
-            cudaGraphDestroy(g);
-            if (ce != cudaSuccess)
-                return fail(SYMGB_ERR_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(ce));
-            u->graphValid = true;
-            u->graphDirect = u->lastRunDirect;
+    bool graph = u->sched.use_graph ||
+                 (u->ranBefore && u->launchesPerRun >= kGraphLaunches && !capturing && !u->graphFailed);
+    if (graph && !u->graphValid) {
+        // The caller did not ask for it: where no graph can be made the launches do.
+        if (int e = makeGraph(u)) {
+            if (u->sched.use_graph) return e;
+            cudaGetLastError();
+            u->graphFailed = true;
+            graph = false;
         }
+    }
+    if (graph) {
         SYMGB_CUDA(cudaGraphLaunch(u->graph, u->stream));
         u->lastRunDirect = u->graphDirect;
         u->lastLaunches = u->launchesPerRun;

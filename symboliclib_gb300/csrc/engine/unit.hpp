@@ -23,6 +23,16 @@ namespace engine {
 // returns `code`.
 int setLastError(int code, const std::string& msg);
 
+// While one lives, what this thread does to its own graphs (instantiation and
+// release allocate and free) does not break a capture that is under way on a
+// stream of the caller's, in whichever mode.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    RelaxedCapture(const RelaxedCapture&) = delete;
+};
+
 struct HostKernel {
     symgb_kernel_desc desc;
     std::vector<symgb_node> nodes;
@@ -129,11 +139,11 @@ struct symgb_unit {
     int tilesSets = -1, tilesItems = -1, tilesMath = -1;
     // One run as a graph (runAsync), until the configuration changes:
     // graphDirect is lastRunDirect after it, ranBefore whether the configuration
-    // has run launch by launch.
+    // has run launch by launch, graphFailed whether a graph of it could not be made.
     // `beside`: kernels that may run beside earlier ones (besideEarlier).
     std::vector<char> beside;
     cudaGraphExec_t graph = nullptr;
-    bool graphValid = false, graphDirect = false, ranBefore = false;
+    bool graphValid = false, graphDirect = false, ranBefore = false, graphFailed = false;
     // Compiled executor: modules by configuration key (schedule kind, math,
     // value sets, block sizes); `current` is the current configuration's, once
     // it has been looked up.
@@ -149,9 +159,12 @@ struct symgb_unit {
     // Forgets what was made for the current configuration (a graph in flight is
     // freed when it completes).
     void dropGraph() {
-        if (graph) cudaGraphExecDestroy(graph);
+        if (graph) {
+            symgb::engine::RelaxedCapture relaxed;
+            cudaGraphExecDestroy(graph);
+        }
         graph = nullptr;
-        graphValid = ranBefore = false;
+        graphValid = ranBefore = graphFailed = false;
         current.reset();
     }
 
