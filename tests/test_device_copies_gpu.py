@@ -60,3 +60,38 @@ def test_page_locked_memory_of_the_host():
     native.check(lib.symgb_get_result_sets_device(u.handle, C.c_void_p(out.data_ptr()), 0))
     native.check(lib.symgb_synchronize(u.handle))
     assert np.array_equal(out.numpy().view(np.uint64), ref.view(np.uint64))
+
+
+@pytest.mark.parametrize("sets", [1, 3, 9])
+def test_inputs_made_on_another_stream(sets):
+    """The unit's stream waits for an event behind which another stream writes
+    the inputs, late; the copy launched after that wait, though chained to what
+    precedes it, takes the new values."""
+    torch = pytest.importorskip("torch")
+    lib = native.symgb()
+    w = native.Workload("cotan", 8, 7)
+    rng = np.random.default_rng(sets)
+    u = native.Unit.from_workload(w)
+    u.set_schedule(kind=native.SCHEDULE_LEVELS, math=native.MATH_EXACT)
+    u.set_num_sets(sets)
+    other, own = torch.cuda.Stream(), torch.cuda.Stream()
+    native.check(lib.symgb_set_stream(u.handle, C.c_void_p(own.cuda_stream)))
+    a = torch.zeros(u.arg_length[0] * sets, dtype=torch.float64, device="cuda")
+    out = torch.zeros(u.output_length[0] * sets, dtype=torch.float64, device="cuda")
+    for _ in range(8):
+        ins = [w.inputs[0] * (1 + 1e-3 * rng.uniform(-1, 1, a.numel() // sets)) for _ in range(sets)]
+        ref = np.concatenate([ocpu.evaluate(w.plan, w.index_data, w.out_index_data, w.const_data, [i])[0] for i in ins])
+        new = torch.from_numpy(np.concatenate(ins)).cuda()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(other):
+            torch.cuda._sleep(1000000)  # half a millisecond
+            a.copy_(new)
+            done = other.record_event()
+        with torch.cuda.stream(own):
+            out.zero_()
+            own.wait_event(done)
+        native.check(lib.symgb_set_arg_sets_device(u.handle, C.c_void_p(a.data_ptr()), 0))
+        native.check(lib.symgb_run_async(u.handle))
+        native.check(lib.symgb_get_result_sets_device(u.handle, C.c_void_p(out.data_ptr()), 0))
+        native.check(lib.symgb_synchronize(u.handle))
+        assert np.array_equal(out.cpu().numpy().view(np.uint64), ref.view(np.uint64))
