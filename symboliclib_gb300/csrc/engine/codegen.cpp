@@ -516,6 +516,7 @@ std::vector<std::vector<Piece>> templatePieces(const std::vector<symgb_kernel_de
     std::vector<int> costs(descs.size(), 0);
     for (std::size_t k = 0; k < descs.size(); ++k) {
         if (!descs[k].num_instances || intMuls[k]) continue;
+        if (!cfg.inPlace.empty() && cfg.inPlace[k]) continue;  // a piece would read what another has stored
         for (const LinOp& L : linearCode(descs[k], cfg.math, nullptr)) costs[k] += fp64Cost(L.op);
         if (costs[k] >= kHeavy) heavy[descs[k].level].push_back((int)k);
     }
@@ -720,38 +721,51 @@ GroupedTables groupedTables(const std::vector<symgb_kernel_desc>& descs) {
     return t;
 }
 
-std::vector<char> besideEarlier(const std::vector<symgb_kernel_desc>& descs, const std::uint32_t* index,
-                                const std::vector<std::uint64_t>& readLo, const std::vector<std::uint64_t>& readHi) {
-    using Range = std::pair<std::uint64_t, std::uint64_t>;  // [first, second)
-    auto writes = [&](std::size_t k) {
-        const symgb_kernel_desc& d = descs[k];
-        return Range(d.output_offset, d.output_offset + d.num_instances * d.num_output_rows);
-    };
-    auto overlap = [](const Range& a, const Range& b) { return std::max(a.first, b.first) < std::min(a.second, b.second); };
-    // The bounds of a kernel's reads settle it for plans in memory order; the
-    // table is only searched where they reach into `r`.
-    auto readsFrom = [&](std::size_t k, const Range& r) {
-        if (readLo[k] > readHi[k] || !overlap(Range(readLo[k], readHi[k] + 1), r)) return false;
-        const symgb_kernel_desc& d = descs[k];
-        for (std::uint32_t a = 0; a < d.num_access; ++a) {
-            const std::uint32_t* row = index + d.index_offset + (std::uint64_t)d.access[2 * a] * d.num_instances;
-            const long long offset = d.access[2 * a + 1];
-            for (std::uint64_t i = 0; i < d.num_instances; ++i) {
-                const std::uint64_t slot = (std::uint64_t)((long long)row[i] + offset);
-                if (slot >= r.first && slot < r.second) return true;
-            }
+namespace {
+
+bool overlap(const SlotUse::Range& a, const SlotUse::Range& b) {
+    return std::max(a.first, b.first) < std::min(a.second, b.second);
+}
+
+}  // namespace
+
+SlotUse::Range SlotUse::writes(std::size_t k) const {
+    const symgb_kernel_desc& d = descs[k];
+    return Range(d.output_offset, d.output_offset + d.num_instances * d.num_output_rows);
+}
+
+// The bounds of a kernel's reads settle it for plans in memory order; the table
+// is only searched where they reach into `r`.
+bool SlotUse::reads(std::size_t k, const Range& r) const {
+    if (readLo[k] > readHi[k] || !overlap(Range(readLo[k], readHi[k] + 1), r)) return false;
+    const symgb_kernel_desc& d = descs[k];
+    for (std::uint32_t a = 0; a < d.num_access; ++a) {
+        const std::uint32_t* row = index + d.index_offset + (std::uint64_t)d.access[2 * a] * d.num_instances;
+        const long long offset = d.access[2 * a + 1];
+        for (std::uint64_t i = 0; i < d.num_instances; ++i) {
+            const std::uint64_t slot = (std::uint64_t)((long long)row[i] + offset);
+            if (slot >= r.first && slot < r.second) return true;
         }
-        return false;
-    };
-    std::vector<char> beside(descs.size(), 0);
+    }
+    return false;
+}
+
+std::vector<char> readsOwnRows(const SlotUse& use) {
+    std::vector<char> own;
+    for (std::size_t k = 0; k < use.descs.size(); ++k) own.push_back(use.reads(k, use.writes(k)));
+    return own;
+}
+
+std::vector<char> besideEarlier(const SlotUse& use) {
+    std::vector<char> beside(use.descs.size(), 0);
     std::vector<std::size_t> group;
-    std::vector<Range> written;  // by the group, adjoining ranges merged
-    for (std::size_t k = 0; k < descs.size(); ++k) {
-        if (!descs[k].num_instances) continue;
-        const Range w = writes(k);
+    std::vector<SlotUse::Range> written;  // by the group, adjoining ranges merged
+    for (std::size_t k = 0; k < use.descs.size(); ++k) {
+        if (!use.descs[k].num_instances) continue;
+        const SlotUse::Range w = use.writes(k);
         bool free = !group.empty();
-        for (std::size_t j = 0; j < written.size() && free; ++j) free = !overlap(w, written[j]) && !readsFrom(k, written[j]);
-        for (std::size_t j = 0; j < group.size() && free; ++j) free = !readsFrom(group[j], w);
+        for (std::size_t j = 0; j < written.size() && free; ++j) free = !overlap(w, written[j]) && !use.reads(k, written[j]);
+        for (std::size_t j = 0; j < group.size() && free; ++j) free = !use.reads(group[j], w);
         if (!free) {
             group.clear();
             written.clear();
@@ -813,7 +827,9 @@ JitSource generateModule(const std::vector<symgb_kernel_desc>& descs, int numLev
     // their own: in one, their compile time grows with its square (Neo-Hookean
     // levels, nine templates of 600 operations: 4.9 -> 1.3 s).
     constexpr std::size_t kHeavyOps = 200;
-    const std::vector<int> intMuls = grouped ? std::vector<int>(descs.size(), 0) : integerProducts(descs, cfg.math, S);
+    std::vector<int> intMuls = grouped ? std::vector<int>(descs.size(), 0) : integerProducts(descs, cfg.math, S);
+    for (std::size_t k = 0; k < cfg.inPlace.size(); ++k)
+        if (cfg.inPlace[k]) intMuls[k] = 0;  // an item evaluated again would read what it has stored
     std::vector<std::vector<Piece>> pieces(descs.size());
     if (!grouped) pieces = templatePieces(descs, cfg, intMuls);
     std::vector<std::size_t> templateOps;

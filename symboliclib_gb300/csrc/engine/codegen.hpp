@@ -7,6 +7,7 @@
 #include <cstdint>
 #include <memory>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "symgb.h"
@@ -35,6 +36,10 @@ struct JitConfig {
     // row's start in the result-position table `dp` - the row's results go to
     // res[dp[start + i]] instead of x - or -1; empty when none is direct.
     std::vector<std::vector<std::int64_t>> directBase;
+    // Per kernel: it reads slots of its own output rows (readsOwnRows), so that
+    // a thread has to read everything before it stores anything, once; empty:
+    // none does.
+    std::vector<char> inPlace;
 };
 
 // Grouped item layout (SYMGB_ITEMS_GROUPED): copies of the index and constant
@@ -72,13 +77,25 @@ struct JitSource {
 // std::runtime_error for templates it cannot express).
 JitSource generateModule(const std::vector<symgb_kernel_desc>& descs, int numLevels, const JitConfig& cfg);
 
+// What the kernels of a plan read and write, from the tables.  readLo[k],
+// readHi[k]: least and greatest slot kernel k reads (lo > hi: none).
+struct SlotUse {
+    const std::vector<symgb_kernel_desc>& descs;
+    const std::uint32_t* index;
+    const std::vector<std::uint64_t>&readLo, &readHi;
+    using Range = std::pair<std::uint64_t, std::uint64_t>;  // [first, second)
+    Range writes(std::size_t k) const;
+    bool reads(std::size_t k, const Range& r) const;
+};
+
+// Which kernels read slots that they write themselves (JitConfig::inPlace).
+std::vector<char> readsOwnRows(const SlotUse& use);
+
 // Which kernels of a plan may run beside those in front of them, in plan order
 // (JIT_PLAIN): [k] is true where kernel k and the kernels back to the last one
 // with false neither read nor write a slot that another of them writes.
 // From the tables alone, so that a plan's level numbers need not be right.
-// readLo[k], readHi[k]: least and greatest slot kernel k reads (lo > hi: none).
-std::vector<char> besideEarlier(const std::vector<symgb_kernel_desc>& descs, const std::uint32_t* index,
-                                const std::vector<std::uint64_t>& readLo, const std::vector<std::uint64_t>& readHi);
+std::vector<char> besideEarlier(const SlotUse& use);
 
 // A compiled and loaded module (jit.cu).  `kernels[j]` is the cudaKernel_t
 // of launches[j], stored as void* (the form the runtime's launch calls take).

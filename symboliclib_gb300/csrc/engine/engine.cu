@@ -374,6 +374,7 @@ JitConfig jitConfig(const symgb_unit* u, int kind) {
     c.minBlocks = std::max(0, u->sched.blocks_per_sm);
     c.loadPath = u->loadPath;
     c.itemLayout = u->itemLayout;
+    c.inPlace = u->inPlace;
     if (u->directOutputs && u->numSets == 1 && u->directRows) c.directBase = u->directBase;
     for (std::size_t k = 0; k < u->kernels.size(); ++k) {
         c.kernelTpb.push_back(u->shapeOf(k).tpb);
@@ -926,7 +927,9 @@ int symgb_init(symgb_unit_t u, const uint32_t* index_data, const uint32_t* out_i
         if (out_index_data[j] >= u->numTotalMemory) return fail(SYMGB_ERR_ARGUMENT, "output id outside x");
     u->release();
     u->jitModules.clear();  // their direct result rows belong to the previous tables
-    u->beside = symgb::engine::besideEarlier(descs, index_data, readLo, readHi);
+    const SlotUse use{descs, index_data, readLo, readHi};
+    u->beside = besideEarlier(use);
+    u->inPlace = readsOwnRows(use);
     // Direct result plan: an output row is direct when each of its slots is
     // read by no kernel and is the slot of exactly one result position
     // (positions are 32-bit in the table: larger result sets are gathered).

@@ -140,10 +140,11 @@ struct symgb_unit {
     // One run as a graph (runAsync), until the configuration changes:
     // graphDirect is lastRunDirect after it, ranBefore whether the configuration
     // has run launch by launch, graphFailed whether a graph of it could not be made.
-    // `beside`: kernels that may run beside earlier ones (besideEarlier).
-    std::vector<char> beside;
     cudaGraphExec_t graph = nullptr;
     bool graphValid = false, graphDirect = false, ranBefore = false, graphFailed = false;
+    // Kernels that may run beside earlier ones (besideEarlier) and kernels that
+    // read slots of their own rows (readsOwnRows), known from init on.
+    std::vector<char> beside, inPlace;
     // Compiled executor: modules by configuration key (schedule kind, math,
     // value sets, block sizes); `current` is the current configuration's, once
     // it has been looked up.

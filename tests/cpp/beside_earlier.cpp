@@ -1,6 +1,6 @@
-// besideEarlier (codegen.hpp) against its definition: slot sets of every
-// kernel, compared pairwise, on random plans whose rows overlap, repeat and
-// point anywhere, and on plans in memory order.
+// besideEarlier and readsOwnRows (codegen.hpp) against their definitions: slot
+// sets of every kernel, compared pairwise, on random plans whose rows overlap,
+// repeat and point anywhere, and on plans in memory order.
 #include <cstdio>
 #include <random>
 #include <set>
@@ -12,7 +12,7 @@ using namespace symgb::engine;
 int main() {
     std::mt19937 rng(5);
     auto pick = [&](int lo, int hi) { return lo + (int)(rng() % (unsigned)(hi - lo + 1)); };
-    int wrong = 0, besides = 0, alone = 0;
+    int wrong = 0, besides = 0, alone = 0, inPlace = 0;
     for (int trial = 0; trial < 20000; ++trial) {
         const bool ordered = trial % 2;  // outputs laid out in plan order, as the front end does
         const int slots = pick(8, 60), kernels = pick(1, 7);
@@ -52,12 +52,18 @@ int main() {
                     hi[k] = std::max(hi[k], (std::uint64_t)s);
                 }
         }
-        const std::vector<char> got = besideEarlier(descs, index.data(), lo, hi);
+        const SlotUse use{descs, index.data(), lo, hi};
+        const std::vector<char> got = besideEarlier(use), own = readsOwnRows(use);
         auto meet = [](const std::set<long long>& a, const std::set<long long>& b) {
             for (long long s : a)
                 if (b.count(s)) return true;
             return false;
         };
+        for (int k = 0; k < kernels; ++k) {
+            const bool expected = meet(reads[k], writes[k]);
+            inPlace += expected;
+            if ((bool)own[k] != expected && ++wrong < 5) std::printf("trial %d kernel %d reads its own rows: %d\n", trial, k, (int)own[k]);
+        }
         std::vector<int> group;
         for (int k = 0; k < kernels; ++k) {
             if (!descs[k].num_instances) continue;
@@ -72,6 +78,6 @@ int main() {
             }
         }
     }
-    std::printf("%d beside, %d not, %d wrong\n", besides, alone, wrong);
-    return wrong || !besides || !alone;
+    std::printf("%d beside, %d not, %d in place, %d wrong\n", besides, alone, inPlace, wrong);
+    return wrong || !besides || !alone || !inPlace;
 }
