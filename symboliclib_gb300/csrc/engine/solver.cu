@@ -677,11 +677,12 @@ int symgb_solver_set_block_preconditioner(symgb_solver_t s, int block_size, int6
     return SYMGB_OK;
 }
 
-// Values of every system, sets innermost.
-static void place(symgb_solver_t s, const double* values, cudaStream_t st) {
-    if (!s->nnzIn) return;
+// Values of every system, sets innermost; a matrix without entries is refused.
+static int place(symgb_solver_t s, const double* values, cudaStream_t st) {
+    if (!s->nnzIn) return symgb::engine::setLastError(SYMGB_ERR_CUDA, "solver: the matrix has no entries");
     const dim3 grid((unsigned)((s->nnzIn + kEntryTile - 1) / kEntryTile), (s->S + kSetTile - 1) / kSetTile);
     placeValues<<<grid, kThreads, 0, st>>>(values, s->nnzIn, s->shared ? nullptr : s->dst.ptr, s->S, s->vals.ptr);
+    return SYMGB_OK;
 }
 
 // y = A z with its dot products (spmv).  Threads to a row: 8 / S while the
@@ -732,7 +733,7 @@ int symgb_solver_multiply(symgb_solver_t s, const double* values, const double* 
     if (!s || !values || !p_dev || !q_dev) return setLastError(SYMGB_ERR_ARGUMENT, "solver: null argument");
     cudaStream_t st = (cudaStream_t)stream;
     const std::uint64_t work = s->n * s->S;
-    place(s, values, st);
+    if (int e = place(s, values, st)) return e;
     // p_dev and q_dev are [set][row]; the same transpose kernel with the roles
     // of rows and sets swapped gives the [row][set] copy of p.
     transposeSets<<<blocksFor(work), kThreads, 0, st>>>(p_dev, s->S, (unsigned)s->n, s->p.ptr);
@@ -758,7 +759,7 @@ static int solveCg(symgb_solver_t s, const double* values, const double* b_dev, 
     double* bb = rr + S;
     const unsigned grid = s->vectorBlocks(s->n), block = s->threads;
     const std::size_t smem = s->sharedBytes();
-    place(s, values, st);
+    if (int e = place(s, values, st)) return e;
     cudaMemsetAsync(s->scalars.ptr, 0, 8 * (std::size_t)S * sizeof(double), st);
     cgStart<<<grid, block, smem, st>>>(b_dev, s->vals.ptr, s->diagPos.ptr, s->n, S, s->x.ptr, s->r.ptr, s->p.ptr,
                                        s->invDiag.ptr, rz, bb);
@@ -813,7 +814,7 @@ static int solveBicgstab(symgb_solver_t s, const double* values, const double* b
     double* omega = alpha + S;
     const unsigned grid = s->vectorBlocks(s->n), block = s->threads;
     const std::size_t smem = s->sharedBytes();
-    place(s, values, st);
+    if (int e = place(s, values, st)) return e;
     cudaMemsetAsync(s->scalars.ptr, 0, 16 * (std::size_t)S * sizeof(double), st);
     bStart<<<grid, block, smem, st>>>(b_dev, s->vals.ptr, s->diagPos.ptr, s->n, S, s->x.ptr, s->r.ptr, s->rhat.ptr,
                                       s->p.ptr, s->v.ptr, s->invDiag.ptr, R, R + S, alpha, omega, bb);

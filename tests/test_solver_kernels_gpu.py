@@ -131,3 +131,15 @@ def test_systems_that_are_not_finite_are_not_reported_as_solved(method, where):
     for s in set(range(sets)) - set(bad):
         ref = np.linalg.solve(dense(n, cp, ri, v[s], True), b[s])
         assert np.linalg.norm(x[s].cpu().numpy() - ref) <= 1e-11 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("sets", [1, 4])
+def test_matrices_without_entries_are_refused(sets):
+    torch = pytest.importorskip("torch")
+    solver = native.SparseSolver(3, np.zeros(4, np.int64), np.zeros(0, np.int32), False, sets)
+    v, b = torch.zeros(1, dtype=torch.float64, device="cuda"), torch.ones((sets, 3), dtype=torch.float64, device="cuda")
+    with pytest.raises(RuntimeError):
+        solver.multiply(v, b, torch.empty_like(b))
+    for method in (native.SOLVER_CG, native.SOLVER_BICGSTAB):
+        with pytest.raises(RuntimeError):
+            solver.solve(v, b, torch.empty_like(b), tol=1e-12, max_iter=16, method=method)
