@@ -26,7 +26,7 @@
 // them, so nothing else is launched.  Figures (GB300, cloth pattern
 // 100 x 100: 30 k rows, 1.14 M entries): BiCGSTAB with 3 x 3 blocks, 8 sets, 143
 // us an iteration with nine launches, two cleared buffers and an atomic
-// addition per row, 66 so; CG, 8 sets, 69 -> 35; CG, one set, 65 -> 17.
+// addition per row, 65 so; CG, 8 sets, 69 -> 34; CG, one set, 65 -> 17.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -689,14 +689,15 @@ static int place(symgb_solver_t s, const double* values, cudaStream_t st) {
 // sets alone would leave a warp's reads scattered over its 32 rows; more, up
 // to a warp, while the threads fill less than half the chip (rows of 39 entries,
 // BiCGSTAB, 4800 rows x 8 sets: 36 us an iteration with one, 28 with four).
-// Only rows shared by lanes need a power of two of threads: 18.7 k rows x 5
-// sets take 40.9 us a CG iteration with 8 threads to a row, 28.1 with 5.
+// Lanes add up by warp shuffles, so only rows shared by lanes need a power of
+// two of threads (18.7 k rows x 5 sets take 40.9 us a CG iteration with 8 threads
+// to a row, 28.1 with 5), and on systems that fill the chip set counts that are
+// none take one thread to a row and set.
 static void product(symgb_solver_t s, const double* z, const double* w, double* y, double* d1, double* d2, double* zero,
                     double* zero2, cudaStream_t st) {
     unsigned width = 1;
     while (width < s->S) width *= 2;
-    unsigned lanes = std::max(1u, 8 / width);
-    if (s->S == 3) lanes = 1;
+    unsigned lanes = width == s->S ? std::max(1u, 8 / width) : 1;
     const std::uint64_t room = (std::uint64_t)s->smCount * 1024;
     const bool wide = width * lanes <= 32 && s->n * width * lanes <= room;
     while (wide && width * lanes < 32 && s->n * width * lanes * 2 <= room) lanes *= 2;
