@@ -141,18 +141,18 @@ class ClockSampler:
                 "reasons": reasons, "samples": len(rows)}
 
 
-# Per-step DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum over the
-# step's launches) from ncu captures of the compiled executor on a GB300,
-# summarised (with their commands) in profiles/.  Keyed by (workload, size, value sets, schedule kind, threads per
+# DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) of the present
+# kernels, per step and of the dominant kernel's launch, from ncu captures of
+# the compiled executor on a GB300, summarised (with their commands) in
+# profiles/.  Keyed by (workload, size, value sets, schedule kind, threads per
 # block, items per thread, minimum CTAs per SM); configurations not captured
 # report null.
 MEASURED = {
-    ("cotan", 500, 1, "levels", 128, 1, 0): {"traffic": 81.77e6, "profile": "profiles/symgb_cotan500_levels.md"},
+    ("cotan", 500, 1, "levels", 128, 1, 0): {"traffic": 88.76e6, "profile": "profiles/symgb_cotan500_levels.md"},
     # full size, single-pass captures: symgb_k1 (the face-block template)
-    # 389.07 MB read + 8.18 GB written per launch; the step's 18 kernels
-    # 18.707 GB
-    ("cloth", 300, 64, "plain", 64, 4, 0): {"kernel_traffic": 8.569e9, "traffic": 18.707e9,
-                                            "profile": "profiles/traffic_cloth300x64_plain.md"},
+    # 428.9 MB read + 9.02 GB written per launch; the step's 18 kernels 19.59 GB
+    ("cloth", 300, 64, "plain", 128, 4, 0): {"kernel_traffic": 9.450e9, "traffic": 19.592e9,
+                                             "profile": "profiles/traffic_cloth300x64_plain.md"},
 }
 
 
@@ -469,7 +469,10 @@ def main_engine(args):
                          "algorithmic_bytes_per_launch": k_bytes, "ms_per_launch": t_k * 1e3,
                          "launches_per_step": 1, "share_of_step": t_k / t_step,
                          "fp64_instructions_per_launch": k_fp64,
-                         "fp64_pipe_frac": k_fp64 / t_k / (fp64.value / 2),
+                         "fp64_instruction_frac": k_fp64 / t_k / (fp64.value / 2),
+                         "fp64_instruction_note": "FP64 instructions of the program / launch time / the measured FMA "
+                                                  "rate; not the pipe's load, as integer pipes take some of the "
+                                                  "products where it fills the chip",
                          "timing": "CUDA events around every kernel on the unit's stream, plain launches of the "
                                    "chosen shape, as many steps as the timed region, L2 cleared before each",
                          "bytes_note": "every gathered value and every result once per value set, index and "
