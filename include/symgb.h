@@ -161,9 +161,10 @@ int symgb_compile_check(symgb_unit_t u, int kind, double* seconds);
 int symgb_compiled_registers(symgb_unit_t u, int kind, int* registers, int cap);
 
 /* Data path of the compiled executor's loads (index and constant tables and
- * the x gathers): the read-only path (ld.global.nc, the default), cached in
- * L1 (ld.global.ca) or in L2 only (ld.global.cg).  Values are the same; the
- * choice changes which load queue the gathers wait in. */
+ * the x gathers): the read-only path (ld.global.nc, the default) for the
+ * tables with the gathers cached in L1, everything cached in L1 (ld.global.ca)
+ * or in L2 only (ld.global.cg).  Values are the same; the choice changes which
+ * load queue the loads wait in. */
 #define SYMGB_LOAD_READONLY 0
 #define SYMGB_LOAD_L1 1
 #define SYMGB_LOAD_L2 2

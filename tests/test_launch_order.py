@@ -69,6 +69,19 @@ def test_copy_kernels_read_what_may_change_with_ordinary_loads():
     assert found >= 5
 
 
+@pytest.mark.parametrize("kind", [PLAIN, LEVELS, PERSISTENT])
+@pytest.mark.parametrize("path", [native.LOAD_READONLY, native.LOAD_L1, native.LOAD_L2])
+def test_generated_kernels_read_x_with_ordinary_loads(path, kind):
+    """x is written while a chained launch is already resident, so no load path
+    reads it through the read-only path."""
+    u = native.Unit.from_workload(workload("cloth", 8), init=False)
+    u.set_load_path(path)
+    src = u.compiled_source(kind)
+    load = re.search(r"double symgbLoadX\(const double\* a\) \{\n(.*?)\n}", src, re.S).group(1)
+    assert load.strip() == f"return L2 ? __ldcg(a) : {'__ldcg' if path == native.LOAD_L2 else '__ldca'}(a);"
+    assert not re.search(r"(SYMGB_LD|__ldg)\(x\b", src)
+
+
 def test_side_by_side_kernels_share_no_written_slot():
     out, lib = build.OBJ / "beside_earlier_test", build.LIB
     subprocess.run(["g++", "-std=c++17", "-O1", f"-I{ROOT / 'include'}", f"-I{build.CSRC / 'engine'}",
