@@ -799,9 +799,9 @@ JitSource generateModule(const std::vector<symgb_kernel_desc>& descs, int numLev
     // earlier in the same launch (L2 = 1) always come from L2.  The read-only
     // path is for the tables alone: a chained launch is resident, waiting, while the
     // one before it still writes x, and that path is for what does not change
-    // while a kernel is resident.  GB300, us with x through it and without:
-    // cotan 100 x 100 11.45 / 11.45, cloth 64 x 64 44.08 / 44.08, 100 x 100 x 64 1568 / 1569;
-    // of others drawn at random two of five lost 1.2 and 1.4 %, none gained.
+    // while a kernel is resident.  GB300, x through it and without: cotan
+    // 100 x 100 11.45 / 11.45 us, cloth 64 x 64 44.08 / 44.08, 300 x 300 x 64 12.64 / 12.68 ms;
+    // of five others drawn at random two lost 1.2 and 1.4 %.
     static const char* const kLoad[] = {"__ldg", "__ldca", "__ldcg"};
     static const char* const kLoadX[] = {"__ldca", "__ldca", "__ldcg"};
     if (cfg.loadPath < 0 || cfg.loadPath > 2) throw std::runtime_error("codegen: load path must be 0, 1 or 2");
